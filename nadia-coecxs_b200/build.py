@@ -2,8 +2,8 @@
 
 Usage: python nadia-coecxs_b200/build.py [--force]
 
-Every .cu file is compiled by nvcc for sm_100a only; plain64.cu additionally
-with --fmad=false so the FP64 path performs no contracted multiply-adds.  The
+Every .cu file is compiled by nvcc for sm_100a only; the FP64 path's files
+additionally with --fmad=false so it performs no contracted multiply-adds.  The
 shared library lands next to this file and is what the Python binding and the
 C++ drop-in headers load.
 """
@@ -26,6 +26,11 @@ PER_FILE = {
     "plain64.cu": ["--fmad=false"],
     "phase_diverse.cu": ["--fmad=false"],
 }
+
+
+def flags(src):
+    # the FP64 transforms: fft64.cu, fft64_p2_*.cu, fft64_any*.cu
+    return ["--fmad=false"] if src.startswith("fft64") else PER_FILE.get(src, [])
 
 
 def sources():
@@ -58,7 +63,7 @@ def build(force=False, verbose=False):
                 and os.path.getmtime(obj) >= hdr_time):
             continue
         lang = [] if src.endswith(".cu") else ["-x", "cu"]
-        jobs.append([NVCC, *COMMON, *PER_FILE.get(src, []), *lang, "-c", path, "-o", obj])
+        jobs.append([NVCC, *COMMON, *flags(src), *lang, "-c", path, "-o", obj])
     with concurrent.futures.ThreadPoolExecutor(max_workers=os.cpu_count() or 4) as pool:
         for out in pool.map(_run, jobs):
             if verbose and out.strip():

@@ -1,0 +1,24 @@
+// fft64_p2_4096.cu -- FP64 transforms of 4096 points.
+#include "fft64_p2.cuh"
+
+namespace nadia {
+namespace plain {
+
+bool rows_p2_4096(int L, RowMode mode, bool fwd, const Fft64Args &A, cudaStream_t st)
+{
+    switch (L) {
+    case 1: return rows_modes<4096, 1>(mode, fwd, A, st);
+    default: return false;
+    }
+}
+
+bool cols_p2_4096(int L, ColMode mode, bool fwd, const Fft64Args &A, cudaStream_t st)
+{
+    switch (L) {
+    case 2: return cols_modes<4096, 2>(mode, fwd, A, st);
+    default: return false;
+    }
+}
+
+} // namespace plain
+} // namespace nadia

@@ -22,219 +22,6 @@ inline int blocks_for(size_t n, int per = kThreads)
     return (int)std::min<size_t>(std::max<size_t>(b, 1), 1u << 30);
 }
 
-__device__ __forceinline__ double2 cmul(double2 a, double2 w)
-{
-    return make_double2(a.x * w.x - a.y * w.y, a.x * w.y + a.y * w.x);
-}
-
-__device__ __forceinline__ void bf4(double2 *v, bool fwd)
-{
-    double2 a, b, c, d;
-    a.x = v[0].x + v[2].x; a.y = v[0].y + v[2].y;
-    b.x = v[0].x - v[2].x; b.y = v[0].y - v[2].y;
-    c.x = v[1].x + v[3].x; c.y = v[1].y + v[3].y;
-    d.x = v[1].x - v[3].x; d.y = v[1].y - v[3].y;
-    v[0].x = a.x + c.x; v[0].y = a.y + c.y;
-    v[2].x = a.x - c.x; v[2].y = a.y - c.y;
-    if (fwd) {
-        v[1].x = b.x + d.y; v[1].y = b.y - d.x;
-        v[3].x = b.x - d.y; v[3].y = b.y + d.x;
-    } else {
-        v[1].x = b.x - d.y; v[1].y = b.y + d.x;
-        v[3].x = b.x + d.y; v[3].y = b.y - d.x;
-    }
-}
-
-__device__ __forceinline__ void bf8(double2 *v, bool fwd)
-{
-    const double c8 = 0.70710678118654752440;
-    double2 a[4], b[4], t;
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        a[r].x = v[r].x + v[r + 4].x; a[r].y = v[r].y + v[r + 4].y;
-        b[r].x = v[r].x - v[r + 4].x; b[r].y = v[r].y - v[r + 4].y;
-    }
-    if (fwd) {
-        t = b[1]; b[1].x = (t.x + t.y) * c8; b[1].y = (t.y - t.x) * c8;
-        t = b[2]; b[2].x = t.y;              b[2].y = -t.x;
-        t = b[3]; b[3].x = (t.y - t.x) * c8; b[3].y = -((t.x + t.y) * c8);
-    } else {
-        t = b[1]; b[1].x = (t.x - t.y) * c8; b[1].y = (t.y + t.x) * c8;
-        t = b[2]; b[2].x = -t.y;             b[2].y = t.x;
-        t = b[3]; b[3].x = -((t.x + t.y) * c8); b[3].y = (t.x - t.y) * c8;
-    }
-    bf4(a, fwd);
-    bf4(b, fwd);
-#pragma unroll
-    for (int r = 0; r < 4; ++r) { v[2 * r] = a[r]; v[2 * r + 1] = b[r]; }
-}
-
-// One Stockham pass of radix R (compile-time for 2/4/8) over L signals of
-// length n held in shared memory (signal stride n).
-template <int R>
-__device__ void pass_fixed(const double2 *src, double2 *dst, int n, int L, int Ns,
-                           const double2 *__restrict__ W, bool fwd)
-{
-    const int m = n / R;
-    const int tstep = n / (Ns * R);
-    for (int b = threadIdx.x; b < L * m; b += blockDim.x) {
-        const int sig = b / m, j = b - sig * m;
-        const double2 *s = src + (size_t)sig * n;
-        double2 *d = dst + (size_t)sig * n;
-        const int k = j % Ns;
-        double2 v[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = s[j + r * m];
-        if (k > 0) {
-#pragma unroll
-            for (int r = 1; r < R; ++r) {
-                double2 w = __ldg(&W[k * r * tstep]);
-                if (!fwd) w.y = -w.y;
-                v[r] = cmul(v[r], w);
-            }
-        }
-        if (R == 2) {
-            double2 a = v[0], c = v[1];
-            v[0].x = a.x + c.x; v[0].y = a.y + c.y;
-            v[1].x = a.x - c.x; v[1].y = a.y - c.y;
-        } else if (R == 4) {
-            bf4(v, fwd);
-        } else {
-            bf8(v, fwd);
-        }
-        const int base = (j / Ns) * Ns * R + k;
-#pragma unroll
-        for (int r = 0; r < R; ++r) d[base + r * Ns] = v[r];
-    }
-}
-
-// Generic (prime) radix: direct sum in increasing r.
-__device__ void pass_generic(const double2 *src, double2 *dst, int n, int L, int R, int Ns,
-                             const double2 *__restrict__ W, bool fwd)
-{
-    const int m = n / R;
-    const int tstep = n / (Ns * R);
-    const int q = n / R;
-    for (int b = threadIdx.x; b < L * m; b += blockDim.x) {
-        const int sig = b / m, j = b - sig * m;
-        const double2 *s = src + (size_t)sig * n;
-        double2 *d = dst + (size_t)sig * n;
-        const int k = j % Ns;
-        if (R > kMaxRadix) {
-            // large primes: the same sums, each twiddled input formed again
-            // from shared memory where it is used (identical arithmetic)
-            auto in = [&](int r) {
-                double2 x = s[j + r * m];
-                if (k > 0 && r > 0) {
-                    double2 w = __ldg(&W[k * r * tstep]);
-                    if (!fwd) w.y = -w.y;
-                    x = cmul(x, w);
-                }
-                return x;
-            };
-            const int base = (j / Ns) * Ns * R + k;
-            double2 y0 = in(0);
-            for (int r = 1; r < R; ++r) {
-                const double2 x = in(r);
-                y0.x = y0.x + x.x;
-                y0.y = y0.y + x.y;
-            }
-            double2 *out0 = d + base;
-            for (int sidx = 1; sidx < R; ++sidx) {
-                double2 acc = in(0);
-                for (int r = 1; r < R; ++r) {
-                    double2 w = __ldg(&W[((r * sidx) % R) * q]);
-                    if (!fwd) w.y = -w.y;
-                    double2 pp = cmul(in(r), w);
-                    acc.x = acc.x + pp.x;
-                    acc.y = acc.y + pp.y;
-                }
-                out0[sidx * Ns] = acc;
-            }
-            out0[0] = y0;
-            continue;
-        }
-        double2 v[kMaxRadix];
-        for (int r = 0; r < R; ++r) v[r] = s[j + r * m];
-        if (k > 0) {
-            for (int r = 1; r < R; ++r) {
-                double2 w = __ldg(&W[k * r * tstep]);
-                if (!fwd) w.y = -w.y;
-                v[r] = cmul(v[r], w);
-            }
-        }
-        const int base = (j / Ns) * Ns * R + k;
-        double2 y0 = v[0];
-        for (int r = 1; r < R; ++r) { y0.x = y0.x + v[r].x; y0.y = y0.y + v[r].y; }
-        d[base] = y0;
-        for (int sidx = 1; sidx < R; ++sidx) {
-            double2 acc = v[0];
-            for (int r = 1; r < R; ++r) {
-                double2 w = __ldg(&W[((r * sidx) % R) * q]);
-                if (!fwd) w.y = -w.y;
-                double2 p = cmul(v[r], w);
-                acc.x = acc.x + p.x; acc.y = acc.y + p.y;
-            }
-            d[base + sidx * Ns] = acc;
-        }
-    }
-}
-
-// All passes of a plan; returns the buffer holding the result.
-__device__ double2 *run_passes(double2 *a, double2 *b, int L, const FftPlan &p,
-                               const double2 *__restrict__ W, bool fwd)
-{
-    int Ns = 1;
-    for (int ip = 0; ip < p.np; ++ip) {
-        const int R = p.radix[ip];
-        if (R == 8)
-            pass_fixed<8>(a, b, p.n, L, Ns, W, fwd);
-        else if (R == 4)
-            pass_fixed<4>(a, b, p.n, L, Ns, W, fwd);
-        else if (R == 2)
-            pass_fixed<2>(a, b, p.n, L, Ns, W, fwd);
-        else
-            pass_generic(a, b, p.n, L, R, Ns, W, fwd);
-        __syncthreads();
-        Ns *= R;
-        double2 *t = a; a = b; b = t;
-    }
-    return a;
-}
-
-__global__ void k_fft_rows(double2 *data, int nx, int ny, int rows, FftPlan p,
-                           const double2 *__restrict__ W, bool fwd)
-{
-    extern __shared__ double2 sm[];
-    double2 *a = sm, *b = sm + (size_t)rows * ny;
-    const int r0 = blockIdx.x * rows;
-    const int nr = min(rows, nx - r0);
-    double2 *g = data + (size_t)r0 * ny;
-    for (int e = threadIdx.x; e < nr * ny; e += blockDim.x) a[e] = g[e];
-    __syncthreads();
-    double2 *res = run_passes(a, b, nr, p, W, fwd);
-    for (int e = threadIdx.x; e < nr * ny; e += blockDim.x) g[e] = res[e];
-}
-
-__global__ void k_fft_cols(double2 *data, int nx, int ny, int cols, FftPlan p,
-                           const double2 *__restrict__ W, bool fwd)
-{
-    extern __shared__ double2 sm[];
-    double2 *a = sm, *b = sm + (size_t)cols * nx;
-    const int c0 = blockIdx.x * cols;
-    const int nc = min(cols, ny - c0);
-    for (int e = threadIdx.x; e < nc * nx; e += blockDim.x) {
-        int i = e / nc, c = e - i * nc;
-        a[(size_t)c * nx + i] = data[(size_t)i * ny + c0 + c];
-    }
-    __syncthreads();
-    double2 *res = run_passes(a, b, nc, p, W, fwd);
-    for (int e = threadIdx.x; e < nc * nx; e += blockDim.x) {
-        int i = e / nc, c = e - i * nc;
-        data[(size_t)i * ny + c0 + c] = res[(size_t)c * nx + i];
-    }
-}
-
 __global__ void k_invert(double2 *a, int nx, int ny, double s)
 {
     const int mx = nx / 2, my = ny / 2;
@@ -312,6 +99,13 @@ __global__ void k_finish_error(const double *partials, int nblocks, double *err)
     if (threadIdx.x == 0) *err = (diff / mag);
 }
 
+// the error metric into the history, as the fused kernels do it themselves
+__global__ void k_record(const double *err, double *ring, int ring_len, long long *iter)
+{
+    ring[*iter % ring_len] = *err;
+    *iter += 1;
+}
+
 __global__ void k_support(double2 *c, const double *__restrict__ sup, size_t n)
 {
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n;
@@ -382,125 +176,6 @@ __global__ void k_combine_support(double2 *x, const double2 *__restrict__ pf,
             vi += W.w[0] * t.y;
         }
         x[k] = make_double2(vr, vi);
-    }
-}
-
-// PlanarCDI's detector side of project_intensity (PlanarCDI.c++:65-73 around
-// BaseCDI::scale_intensity, BaseCDI.c++:163-189) between the two transforms:
-// invert(scale) -> scale_intensity -> invert(scale).  The quadrant swap pairs
-// q with p(q), so per element out[q] = s * set_mag(s * a[q], sqrt(I)[p(q)])
-// (measured pixels; s * (s * a[q]) otherwise) -- the same operations.
-__global__ void k_detector_planar(double2 *c, const double *__restrict__ isqrt,
-                                  const double *__restrict__ bs, int nx, int ny, double s,
-                                  double *partials)
-{
-    double diff = 0, mag = 0;
-    const int mx = nx / 2, my = ny / 2;
-    const size_t n = (size_t)nx * ny;
-    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n;
-         q += (size_t)gridDim.x * blockDim.x) {
-        const int i = (int)(q / ny), j = (int)(q - (size_t)i * ny);
-        const int ip = i < mx ? i + mx : i - mx, jp = j < my ? j + my : j - my;
-        const size_t d = (size_t)ip * ny + jp;
-        const double2 u = c[q];
-        double2 v = make_double2(u.x * s, u.y * s);
-        if (bs == nullptr || bs[d] > 0) {
-            const double cis = isqrt[d];
-            const double cm = mag_of(v);
-            v = set_mag(v, cis);
-            mag += cis * cis;
-            diff += (cm - cis) * (cm - cis);
-        }
-        c[q] = make_double2(v.x * s, v.y * s);
-    }
-    block_sum2(diff, mag);
-    if (threadIdx.x == 0) {
-        partials[2 * blockIdx.x] = diff;
-        partials[2 * blockIdx.x + 1] = mag;
-    }
-}
-
-// FresnelCDI's detector side between the two transforms (FresnelCDI.c++:217-250):
-// multiply_factors(-1) -> add(illumination) -> scale_intensity ->
-// add(-illumination) -> multiply_factors(+1), all at the same element.
-__global__ void k_detector_fresnel(double2 *c, const double2 *__restrict__ coef,
-                                   const double2 *__restrict__ ill,
-                                   const double *__restrict__ isqrt,
-                                   const double *__restrict__ bs, int nx, int ny,
-                                   double *partials)
-{
-    double diff = 0, mag = 0;
-    const double x_mid = (nx - 1) / 2.0, y_mid = (ny - 1) / 2.0;
-    const int qy = ny / 2;
-    const size_t n = (size_t)nx * ny;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n;
-         e += (size_t)gridDim.x * blockDim.x) {
-        const int i = (int)(e / ny), j = (int)(e - (size_t)i * ny);
-        const int i_ = (int)(x_mid - fabs(x_mid - i));
-        const int j_ = (int)(y_mid - fabs(y_mid - j));
-        const double2 cf = coef[(size_t)i_ * qy + j_];
-        const double2 t = ill[e];
-        double2 o = c[e];
-        double cr = cf.x, ci = -1 * cf.y;
-        double2 v = make_double2(o.x * cr - o.y * ci, o.y * cr + o.x * ci);
-        v = make_double2(v.x + 1.0 * t.x, v.y + 1.0 * t.y);
-        if (bs == nullptr || bs[e] > 0) {
-            const double cis = isqrt[e];
-            const double cm = mag_of(v);
-            v = set_mag(v, cis);
-            mag += cis * cis;
-            diff += (cm - cis) * (cm - cis);
-        }
-        v = make_double2(v.x + -1.0 * t.x, v.y + -1.0 * t.y);
-        ci = 1 * cf.y;
-        c[e] = make_double2(v.x * cr - v.y * ci, v.y * cr + v.x * ci);
-    }
-    block_sum2(diff, mag);
-    if (threadIdx.x == 0) {
-        partials[2 * blockIdx.x] = diff;
-        partials[2 * blockIdx.x + 1] = mag;
-    }
-}
-
-// multiply_factors' operation on element (i, j)
-__device__ __forceinline__ double2 factor_at(double2 o, const double2 *__restrict__ coef, int i,
-                                             int j, int nx, int ny, int direction)
-{
-    const double x_mid = (nx - 1) / 2.0, y_mid = (ny - 1) / 2.0;
-    const int i_ = (int)(x_mid - fabs(x_mid - i));
-    const int j_ = (int)(y_mid - fabs(y_mid - j));
-    const double2 cf = coef[(size_t)i_ * (ny / 2) + j_];
-    const double cr = cf.x, ci = direction * cf.y;
-    return make_double2(o.x * cr - o.y * ci, o.y * cr + o.x * ci);
-}
-
-// invert(scale) and multiply_factors in one pass (FresnelCDI_WF.c++:165-182):
-// each thread takes a swap pair (q, p(q)); factors_first multiplies before
-// the swap (propagate_to_detector), otherwise after it (propagate_from)
-__global__ void k_invert_factors(double2 *a, const double2 *__restrict__ coef, int nx, int ny,
-                                 double s, int direction, int factors_first)
-{
-    const int mx = nx / 2, my = ny / 2;
-    const size_t total = (size_t)nx * my;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total;
-         e += (size_t)gridDim.x * blockDim.x) {
-        const int i = (int)(e / my), j = (int)(e - (size_t)i * my);
-        const int jn = j + my;
-        int in = i + mx;
-        if (i >= mx) in = in - 2 * mx;
-        double2 *pp = a + (size_t)in * ny + jn, *qq = a + (size_t)i * ny + j;
-        double2 t = *pp, u = *qq;
-        if (factors_first) {
-            t = factor_at(t, coef, in, jn, nx, ny, direction);
-            u = factor_at(u, coef, i, j, nx, ny, direction);
-        }
-        double2 np = make_double2(u.x * s, u.y * s), nq = make_double2(t.x * s, t.y * s);
-        if (!factors_first) {
-            np = factor_at(np, coef, in, jn, nx, ny, direction);
-            nq = factor_at(nq, coef, i, j, nx, ny, direction);
-        }
-        *pp = np;
-        *qq = nq;
     }
 }
 
@@ -585,6 +260,26 @@ __global__ void k_poly_expand(const double2 *__restrict__ c, const double *__res
             }
         }
         isc[e] = sqrt(acc);
+    }
+}
+
+// expand_wl on the squared magnitudes of the centred field, through the
+// sample rows and columns of each line (set_spectrum forms them as
+// k_poly_expand does; -1: outside)
+__global__ void k_poly_gather(const double *__restrict__ q, const double *__restrict__ spec, int nl,
+                              const int *__restrict__ rows, const int *__restrict__ cols, int nx,
+                              int ny, int my, double *isc)
+{
+    for (int i = blockIdx.y; i < nx; i += gridDim.y) {
+        for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < ny; j += gridDim.x * blockDim.x) {
+            double acc = 0.0;
+            for (int l = 0; l < nl; ++l) {
+                const int r = __ldg(&rows[l * nx + i]), c = __ldg(&cols[l * ny + j]);
+                if (r >= 0 && c >= 0)
+                    acc = acc + __ldg(&spec[2 * l + 1]) * __ldg(&q[(size_t)r * my + c]);
+            }
+            isc[(size_t)i * ny + j] = sqrt(acc);
+        }
     }
 }
 
@@ -760,198 +455,9 @@ __global__ void k_autocorr_fill(const double *__restrict__ isqrt, double2 *t, si
     }
 }
 
-// A pass of radix R (2, 4 or 8) over L signals of length n in ONE shared
-// buffer: every thread loads the inputs of its butterflies (at most EPT
-// elements) into registers, the block synchronises, then each thread applies
-// the twiddles and the butterfly of pass_fixed and stores its outputs.  Same
-// arithmetic as pass_fixed, half its shared memory (twice the resident
-// blocks).  Requires L * n <= EPT * NT.
-template <int R, int EPT, int NT>
-__device__ __forceinline__ void pass_one_buffer(double2 *buf, int n, int L, int Ns,
-                                                const double2 *__restrict__ W, bool fwd)
-{
-    constexpr int NB = EPT / R;
-    const int m = n / R;
-    const int tstep = n / (Ns * R);
-    const int total = L * m;
-    double2 v[NB][R];
-#pragma unroll
-    for (int q = 0; q < NB; ++q) {
-        const int b = threadIdx.x + q * NT;
-        if (b < total) {
-            const int sig = b / m, j = b - sig * m;
-            const double2 *src = buf + (size_t)sig * n;
-#pragma unroll
-            for (int r = 0; r < R; ++r) v[q][r] = src[j + r * m];
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < NB; ++q) {
-        const int b = threadIdx.x + q * NT;
-        if (b < total) {
-            const int sig = b / m, j = b - sig * m;
-            double2 *dst = buf + (size_t)sig * n;
-            const int k = j % Ns;
-            double2 *x = v[q];
-            if (k > 0) {
-#pragma unroll
-                for (int r = 1; r < R; ++r) {
-                    double2 w = __ldg(&W[k * r * tstep]);
-                    if (!fwd) w.y = -w.y;
-                    x[r] = cmul(x[r], w);
-                }
-            }
-            if (R == 2) {
-                double2 a = x[0], c = x[1];
-                x[0].x = a.x + c.x; x[0].y = a.y + c.y;
-                x[1].x = a.x - c.x; x[1].y = a.y - c.y;
-            } else if (R == 4) {
-                bf4(x, fwd);
-            } else {
-                bf8(x, fwd);
-            }
-            const int base = (j / Ns) * Ns * R + k;
-#pragma unroll
-            for (int r = 0; r < R; ++r) dst[base + r * Ns] = x[r];
-        }
-    }
-    __syncthreads();
-}
-
-template <int EPT, int NT>
-__device__ void run_passes_one_buffer(double2 *buf, int L, const FftPlan &p,
-                                      const double2 *__restrict__ W, bool fwd)
-{
-    int Ns = 1;
-    for (int ip = 0; ip < p.np; ++ip) {
-        const int R = p.radix[ip];
-        if (R == 8)
-            pass_one_buffer<8, EPT, NT>(buf, p.n, L, Ns, W, fwd);
-        else if (R == 4)
-            pass_one_buffer<4, EPT, NT>(buf, p.n, L, Ns, W, fwd);
-        else
-            pass_one_buffer<2, EPT, NT>(buf, p.n, L, Ns, W, fwd);
-        Ns *= R;
-    }
-}
-
-template <int EPT, int NT, int MINB>
-__global__ void __launch_bounds__(NT, MINB) k_fft_rows1(double2 *data, int nx, int ny, int rows,
-                                                  FftPlan p, const double2 *__restrict__ W,
-                                                  bool fwd)
-{
-    extern __shared__ double2 sm[];
-    const int r0 = blockIdx.x * rows;
-    const int nr = min(rows, nx - r0);
-    double2 *g = data + (size_t)r0 * ny;
-    for (int e = threadIdx.x; e < nr * ny; e += NT) sm[e] = g[e];
-    __syncthreads();
-    run_passes_one_buffer<EPT, NT>(sm, nr, p, W, fwd);
-    for (int e = threadIdx.x; e < nr * ny; e += NT) g[e] = sm[e];
-}
-
-template <int EPT, int NT, int MINB>
-__global__ void __launch_bounds__(NT, MINB) k_fft_cols1(double2 *data, int nx, int ny, int cols,
-                                                  FftPlan p, const double2 *__restrict__ W,
-                                                  bool fwd)
-{
-    extern __shared__ double2 sm[];
-    const int c0 = blockIdx.x * cols;
-    const int nc = min(cols, ny - c0);
-    for (int e = threadIdx.x; e < nc * nx; e += NT) {
-        int i = e / nc, c = e - i * nc;
-        sm[(size_t)c * nx + i] = data[(size_t)i * ny + c0 + c];
-    }
-    __syncthreads();
-    run_passes_one_buffer<EPT, NT>(sm, nc, p, W, fwd);
-    for (int e = threadIdx.x; e < nc * nx; e += NT) {
-        int i = e / nc, c = e - i * nc;
-        data[(size_t)i * ny + c0 + c] = sm[(size_t)c * nx + i];
-    }
-}
-
-bool pow2_radices(const FftPlan &p)
-{
-    for (int i = 0; i < p.np; ++i)
-        if (p.radix[i] != 2 && p.radix[i] != 4 && p.radix[i] != 8) return false;
-    return true;
-}
-
 inline int grid_of(size_t n) { return std::min(blocks_for(n), 148 * 16); }
 
 } // namespace
-
-// one-buffer kernels: 8 elements per thread; rows with 256 threads (signals
-// of up to 2048 points), columns with 256 threads, or 512 from 2048 points
-constexpr int kRowNT = 256, kRowEPT = 8, kRowMinB = 2, kColNT = 256, kColEPT = 8, kColMinB = 2,
-              kColWideNT = 512;
-
-void Fft2d::init(int nx_, int ny_)
-{
-    nx = nx_;
-    ny = ny_;
-    px = make_plan(nx);
-    py = make_plan(ny);
-    std::vector<double2> hx = twiddles(nx), hy = twiddles(ny);
-    wx.alloc(nx);
-    wy.alloc(ny);
-    upload_now(wx.p, hx.data(), wx.bytes());
-    upload_now(wy.p, hy.data(), wy.bytes());
-    const size_t budget = 128 * 1024;
-    rows_per_block = std::max(1, 2048 / ny);
-    while (rows_per_block > 1 && 2 * (size_t)rows_per_block * ny * sizeof(double2) > budget)
-        --rows_per_block;
-    cols_per_block = std::max(1, std::min(8, 4096 / nx));
-    while (cols_per_block > 1 && 2 * (size_t)cols_per_block * nx * sizeof(double2) > budget)
-        --cols_per_block;
-    // radix-2/4/8 plans run the one-buffer kernels (measured on B200 at
-    // 1024^2 and 2048^2: 10-14% less time per FP64 iteration); columns of
-    // 2048 points and more with 512 threads
-    row_one = pow2_radices(py) && ny <= kRowEPT * kRowNT;
-    if (row_one) rows_per_block = std::max(1, kRowEPT * kRowNT / ny);
-    col_wide = nx >= 2048;
-    const int col_nt = col_wide ? kColWideNT : kColNT;
-    col_one = pow2_radices(px) && nx <= kColEPT * col_nt;
-    if (col_one) cols_per_block = std::max(1, std::min(4, kColEPT * col_nt / nx));
-    row_smem = (row_one ? 1 : 2) * (size_t)rows_per_block * ny * sizeof(double2);
-    col_smem = (col_one ? 1 : 2) * (size_t)cols_per_block * nx * sizeof(double2);
-    NADIA_REQUIRE(row_smem <= 227 * 1024 && col_smem <= 227 * 1024, NADIA_ERR_INVALID,
-                  "grid too large for the FP64 transform");
-    // the attribute belongs to the kernel, not to this plan: every plan sets
-    // the same (largest) limit, so a smaller plan made later cannot lower it
-    // below what an earlier, larger plan launches with
-    NADIA_CUDA(cudaFuncSetAttribute(k_fft_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    227 * 1024));
-    NADIA_CUDA(cudaFuncSetAttribute(k_fft_cols, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    227 * 1024));
-    NADIA_CUDA(cudaFuncSetAttribute(k_fft_rows1<kRowEPT, kRowNT, kRowMinB>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    NADIA_CUDA(cudaFuncSetAttribute(k_fft_cols1<kColEPT, kColNT, kColMinB>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    NADIA_CUDA(cudaFuncSetAttribute(k_fft_cols1<kColEPT, kColWideNT, 1>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-}
-
-void Fft2d::exec(double2 *a, bool forward, cudaStream_t s) const
-{
-    int gr = (nx + rows_per_block - 1) / rows_per_block;
-    if (row_one)
-        k_fft_rows1<kRowEPT, kRowNT, kRowMinB><<<gr, kRowNT, row_smem, s>>>(a, nx, ny, rows_per_block, py,
-                                                                 wy.p, forward);
-    else
-        k_fft_rows<<<gr, kThreads, row_smem, s>>>(a, nx, ny, rows_per_block, py, wy.p, forward);
-    int gc = (ny + cols_per_block - 1) / cols_per_block;
-    if (col_one && col_wide)
-        k_fft_cols1<kColEPT, kColWideNT, 1><<<gc, kColWideNT, col_smem, s>>>(
-            a, nx, ny, cols_per_block, px, wx.p, forward);
-    else if (col_one)
-        k_fft_cols1<kColEPT, kColNT, kColMinB><<<gc, kColNT, col_smem, s>>>(a, nx, ny, cols_per_block, px,
-                                                                 wx.p, forward);
-    else
-        k_fft_cols<<<gc, kThreads, col_smem, s>>>(a, nx, ny, cols_per_block, px, wx.p, forward);
-    NADIA_CUDA(cudaGetLastError());
-}
 
 // Odd grids: Complex_2D::invert's swap loop (Complex_2D.c++:318-353) then
 // visits some elements twice and never moves the last column (for odd ny),
@@ -1049,14 +555,6 @@ void combine(double2 *x, const double2 *pfs, const double2 *pf, const double2 *p
     k_combine<<<grid_of(n), kThreads, 0, s>>>(x, pfs, pf, ps, psf, W, n);
 }
 
-void invert_factors(double2 *c, const double2 *coef, int nx, int ny, int direction,
-                    bool factors_first, cudaStream_t s)
-{
-    const double f = 1.0 / (sqrt((double)(nx * ny)));
-    k_invert_factors<<<grid_of((size_t)nx * (ny / 2)), kThreads, 0, s>>>(
-        c, coef, nx, ny, f, direction, factors_first ? 1 : 0);
-}
-
 void combine_support(double2 *x, const double2 *pf, const double *support, bool use_ps,
                      bool use_psf, const double w[5], size_t n, cudaStream_t s)
 {
@@ -1065,22 +563,6 @@ void combine_support(double2 *x, const double2 *pf, const double *support, bool 
     W.id = 1 + w[4];
     k_combine_support<<<grid_of(n), kThreads, 0, s>>>(x, pf, support, use_ps ? 1 : 0,
                                                      use_psf ? 1 : 0, W, n);
-}
-
-void detector_planar(double2 *c, const double *isqrt, const double *bs, int nx, int ny,
-                     double *partials, double *err, cudaStream_t s)
-{
-    const double f = 1.0 / (sqrt((double)(nx * ny))); // invert(scale), Complex_2D.c++:318-353
-    k_detector_planar<<<kRedBlocks, kThreads, 0, s>>>(c, isqrt, bs, nx, ny, f, partials);
-    k_finish_error<<<1, kThreads, 0, s>>>(partials, kRedBlocks, err);
-}
-
-void detector_fresnel(double2 *c, const double2 *coef, const double2 *ill, const double *isqrt,
-                      const double *bs, int nx, int ny, double *partials, double *err,
-                      cudaStream_t s)
-{
-    k_detector_fresnel<<<kRedBlocks, kThreads, 0, s>>>(c, coef, ill, isqrt, bs, nx, ny, partials);
-    k_finish_error<<<1, kThreads, 0, s>>>(partials, kRedBlocks, err);
 }
 
 void multiply_factors(double2 *c, const double2 *coef, int nx, int ny, int direction,
@@ -1115,6 +597,18 @@ void poly_expand(const double2 *c, const double *spec, int nl, double lambdac, i
 {
     k_poly_expand<<<grid_of((size_t)nx * ny), kThreads, 0, s>>>(c, spec, nl, lambdac, nx, ny,
                                                                px, py, isc);
+}
+
+void poly_gather(const double *q, const double *spec, int nl, const int *rows, const int *cols,
+                 int nx, int ny, int my, double *isc, cudaStream_t s)
+{
+    dim3 grid((ny + 127) / 128, std::min(nx, 65535));
+    k_poly_gather<<<grid, 128, 0, s>>>(q, spec, nl, rows, cols, nx, ny, my, isc);
+}
+
+void record_error(const double *err, double *ring, int ring_len, long long *iter, cudaStream_t s)
+{
+    k_record<<<1, 1, 0, s>>>(err, ring, ring_len, iter);
 }
 
 void poly_scale(double2 *c, const double *isc, const double *isqrt, const double *bs, int nx,

@@ -2,11 +2,14 @@
 // (NADIA/src/Complex_2D.c++, BaseCDI.c++, PlanarCDI.c++, FresnelCDI.c++,
 // PolyCDI.c++), each performing the same sequence of IEEE-754 double
 // operations per element as the reference's double build, so results agree
-// bit for bit except for the order of the error-metric sums.  plain64.cu is
-// compiled with --fmad=false so no multiply-add is contracted.
+// bit for bit except for the order of the error-metric sums.  The steps of an
+// iteration that lie next to a transform run inside it (fft64.h); the kernels
+// here serve everything else.  Compiled with --fmad=false so no multiply-add
+// is contracted.
 #pragma once
 
 #include "common.h"
+#include "fft64.h"
 
 namespace nadia {
 namespace plain {
@@ -14,20 +17,6 @@ namespace plain {
 // Number of blocks used by the two-stage reductions (fixed, so the summation
 // order is the same on every call).
 constexpr int kRedBlocks = 592;
-
-// In-place unnormalised 2-D DFT of an nx-by-ny row-major double2 array with
-// the canonical Stockham schedule: every row (length ny), then every column.
-struct Fft2d {
-    int nx = 0, ny = 0;
-    FftPlan px{}, py{};
-    DevBuf<double2> wx, wy;
-    int rows_per_block = 1, cols_per_block = 1;
-    size_t row_smem = 0, col_smem = 0;
-    bool row_one = false, col_one = false; // radix-2/4/8 plans: the one-buffer kernels
-    bool col_wide = false;                 // columns of 2048 points and more: 512 threads
-    void init(int nx, int ny);
-    void exec(double2 *a, bool forward, cudaStream_t s) const;
-};
 
 // Complex_2D::invert(scale), Complex_2D.c++:318-353 (even sizes).
 // scratch: nx*ny values, needed for odd sizes (the swap loop's replay is a
@@ -53,21 +42,6 @@ void combine(double2 *x, const double2 *pfs, const double2 *pf, const double2 *p
 void combine_support(double2 *x, const double2 *pf, const double *support, bool use_ps,
                      bool use_psf, const double w[5], size_t n, cudaStream_t s);
 
-// The detector side of project_intensity between its two transforms, one
-// kernel each: PlanarCDI invert -> scale_intensity -> invert (PlanarCDI.c++:
-// 65-73); FresnelCDI multiply_factors -> add(W) -> scale_intensity ->
-// add(-W) -> multiply_factors (FresnelCDI.c++:217-250).  Error to *err.
-void detector_planar(double2 *c, const double *isqrt, const double *bs, int nx, int ny,
-                     double *partials, double *err, cudaStream_t s);
-void detector_fresnel(double2 *c, const double2 *coef, const double2 *ill, const double *isqrt,
-                      const double *bs, int nx, int ny, double *partials, double *err,
-                      cudaStream_t s);
-
-// invert(scale) and multiply_factors in one pass, the factors applied before
-// the swap (factors_first) or after it -- FresnelCDI_WF's propagations.
-void invert_factors(double2 *c, const double2 *coef, int nx, int ny, int direction,
-                    bool factors_first, cudaStream_t s);
-
 // FresnelCDI::multiply_factors, FresnelCDI.c++:98-126 (quarter table coef).
 void multiply_factors(double2 *c, const double2 *coef, int nx, int ny, int direction,
                       cudaStream_t s);
@@ -87,6 +61,14 @@ void unpad(const double2 *p, int nx, int ny, int px, int py, double2 *x, cudaStr
 // normalised weight) pairs on the device.
 void poly_expand(const double2 *c, const double *spec, int nlambda, double lambdac, int nx,
                  int ny, int px, int py, double *isqrt_calc, cudaStream_t s);
+
+// The same from the centred field's squared magnitudes q (rows of my values),
+// through per-line tables of sample rows and columns (-1: outside).
+void poly_gather(const double *q, const double *spec, int nlambda, const int *rows,
+                 const int *cols, int nx, int ny, int my, double *isqrt_calc, cudaStream_t s);
+
+// *err into the history: ring[*iter % ring_len], and *iter counted on.
+void record_error(const double *err, double *ring, int ring_len, long long *iter, cudaStream_t s);
 
 // PolyCDI::scale_intensity, PolyCDI.c++:255-292 (c is the padded field).
 void poly_scale(double2 *c, const double *isqrt_calc, const double *isqrt,

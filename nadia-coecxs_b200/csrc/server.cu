@@ -34,18 +34,24 @@ size_t footprint_bytes(int kind, int nx, int ny, int prec, int n_best, int pad_n
     // error value, error history, reduction scratch, maxima (solver.cu)
     size_t b = 8 + 8 * (size_t)Solver::kRing + 8 * (2 * (size_t)plain::kRedBlocks + 64) + 16;
     if (prec == NADIA_FP64) {
+        const size_t m = (size_t)std::max(std::max(nx, ny), std::max(pad_nx, pad_ny));
+        if (m > plain::kRedBlocks) b += 16 * (m - plain::kRedBlocks); // one error pair per block
+        b += 16;                                          // history counter, ticket
         b += n * (16 + 8 + 8 + 8 + 8); // x, support, sqrt(I), blur result, scratch
-        if (kind != NADIA_FRESNEL_WF) b += 4 * 16 * n; // the combine's projection terms at most
+        // the combine's projection terms at most; FresnelCDI_WF's second field
+        b += (kind != NADIA_FRESNEL_WF ? 4 : 1) * 16 * n;
         b += 8 * n;                    // beam stop
-        b += 16 * (size_t)(nx + ny);   // transform twiddles
+        // transform twiddles and the prime radices' tables (a prime factor of
+        // 1021 at most adds as much again)
+        b += 16 * (size_t)(2 * (nx + ny) + 4);
         if ((nx | ny) & 1) b += 16 * n; // odd grids: the quadrant swap's gather target
         b += 8 * 64;                   // blur kernel table
         b += (size_t)n_best * 16 * n;
         if (kind == NADIA_FRESNEL) b += 16 * n + 16 * n + 16 * (size_t)(nx / 2) * (ny / 2);
         if (kind == NADIA_FRESNEL_WF) b += 16 * (size_t)(nx / 2) * (ny / 2);
         if (kind == NADIA_POLY)
-            b += 16 * (size_t)nlambda + 16 * (size_t)pad_nx * pad_ny + 8 * n +
-                 16 * (size_t)(pad_nx + pad_ny);
+            b += 16 * (size_t)nlambda + 24 * (size_t)pad_nx * pad_ny + 8 * n +
+                 4 * (size_t)nlambda * (nx + ny) + 16 * (size_t)(2 * (pad_nx + pad_ny) + 4);
     } else {
         b += n * (8 + 8 + 4 + 4);                     // P, x, support, sqrt(I)
         // partials (one per column tile; FresnelCDI_WF one per row tile),

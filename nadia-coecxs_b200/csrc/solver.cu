@@ -108,6 +108,7 @@ Solver::Solver(int kind_, int nx_, int ny_, int prec_, int n_best_)
     d_err.alloc(1);
     d_ring.alloc(kRing);
     partials.alloc(2 * plain::kRedBlocks + 64);
+    if (prec == NADIA_FP64) plain_counters();
     NADIA_CUDA(cudaMemsetAsync(d_err.p, 0, sizeof(double), st));
     NADIA_CUDA(cudaMemsetAsync(d_ring.p, 0, d_ring.bytes(), st));
     best_err.assign(n_best, 1.0);   // BaseCDI.c++:48
@@ -138,6 +139,24 @@ Solver::Solver(int kind_, int nx_, int ny_, int prec_, int n_best_)
     algorithm = NADIA_CUSTOM;   // BaseCDI.c++:63-64
     set_algorithm(NADIA_ER);
     NADIA_CUDA(cudaStreamSynchronize(st));
+}
+
+// FP64: the history's counter, the error sums' ticket and their partials
+void Solver::plain_counters()
+{
+    plain_partials((size_t)std::max(nx, ny));
+    d_iter.alloc(1);
+    ticket.alloc(1);
+    h2d(d_iter.p, &iters, sizeof(iters), st);
+    NADIA_CUDA(cudaMemsetAsync(ticket.p, 0, sizeof(unsigned), st));
+}
+
+// room for one pair of error sums per block
+void Solver::plain_partials(size_t blocks)
+{
+    if (partials.n >= 2 * blocks + 64) return;
+    NADIA_CUDA(cudaStreamSynchronize(st)); // queued work may still use the old one
+    partials.alloc(2 * blocks + 64);
 }
 
 Solver::~Solver()
@@ -278,9 +297,36 @@ void Solver::set_spectrum(const double *wl_weight, int nl)
         padded.alloc((size_t)(nx + 2 * px) * (ny + 2 * py));
         isc.alloc(n);
         fft_pad.init(nx + 2 * px, ny + 2 * py);
+        poly_tables();
     } else {
         f32->set_spectrum();
     }
+}
+
+// The sample row and column of each line for every measured pixel, in the
+// operation order of expand_wl (PolyCDI.c++:312-318); -1 outside the padded
+// grid.  Rows are kept as offsets into the padded array.
+void Solver::poly_tables()
+{
+    const int mx = nx + 2 * px, my = ny + 2 * py;
+    std::vector<int> r((size_t)nlambda * nx), c((size_t)nlambda * ny);
+    for (int l = 0; l < nlambda; ++l) {
+        const double lf = spectrum[2 * l] / lambdac;
+        for (int i = 0; i < nx; ++i) {
+            const double v = lf * (i + px - nx / 2.0) + nx / 2.0;
+            r[(size_t)l * nx + i] = (v >= 0 && v < mx) ? (int)v : -1;
+        }
+        for (int j = 0; j < ny; ++j) {
+            const double v = lf * (j + py - ny / 2.0) + ny / 2.0;
+            c[(size_t)l * ny + j] = (v >= 0 && v < my) ? (int)v : -1;
+        }
+    }
+    d_rows.alloc(r.size());
+    d_cols.alloc(c.size());
+    d_q.alloc((size_t)mx * my);
+    h2d(d_rows.p, r.data(), d_rows.bytes(), st);
+    h2d(d_cols.p, c.data(), d_cols.bytes(), st);
+    plain_partials((size_t)std::max(mx, my));
 }
 
 void Solver::require_poly_ready() const
@@ -794,6 +840,7 @@ void Solver::convert_to_fp64()
     isqrt.alloc(n);
     recon.alloc(n);
     tmp.alloc(n);
+    plain_counters();
     fft.init(nx, ny);
     gauss_width_ = -1;
     gauss_cut_ = -1;
@@ -823,6 +870,7 @@ void Solver::convert_to_fp64()
         padded.alloc((size_t)(nx + 2 * px) * (ny + 2 * py));
         isc.alloc(n);
         fft_pad.init(nx + 2 * px, ny + 2 * py);
+        poly_tables();
     }
     if (had_tc) set_transmission_constraint(tcu, tcf, tcs, 0, nullptr, nullptr, nullptr);
     NADIA_CUDA(cudaStreamSynchronize(st));
@@ -858,8 +906,17 @@ void Solver::plain_propagate_to(double2 *c, bool pg)
     if (kind == NADIA_FRESNEL_WF) {
         // FresnelCDI_WF::propagate_to_detector, FresnelCDI_WF.c++:176-182
         fft.exec(c, true, st);
-        plain::invert_factors(c, coef.p, nx, ny, -1, true, st); // factors, then the swap
-        fft.exec(c, true, st);
+        plain::Fft64Args A; // factors, then the swap, on the way into the second transform
+        A.src = c;
+        A.dst = second();
+        A.count = nx;
+        A.coef = coef.p;
+        A.s = 1.0 / (sqrt((double)(nx * ny)));
+        fft.rows(plain::R_WF_TO, true, A, st);
+        A.src = A.dst;
+        A.dst = c;
+        A.count = ny;
+        fft.cols(plain::C_PLAIN, true, A, st);
     } else if (kind == NADIA_FRESNEL) {
         // FresnelCDI::propagate_to_detector, FresnelCDI.c++:245-250
         plain::invert(c, nx, ny, true, st);
@@ -882,8 +939,17 @@ void Solver::plain_propagate_from(double2 *c, bool pg)
     if (kind == NADIA_FRESNEL_WF) {
         // FresnelCDI_WF::propagate_from_detector, FresnelCDI_WF.c++:165-173
         fft.exec(c, false, st);
-        plain::invert_factors(c, coef.p, nx, ny, +1, false, st); // the swap, then factors
-        fft.exec(c, false, st);
+        plain::Fft64Args A; // the swap, then factors, on the way into the second transform
+        A.src = c;
+        A.dst = second();
+        A.count = nx;
+        A.coef = coef.p;
+        A.s = 1.0 / (sqrt((double)(nx * ny)));
+        fft.rows(plain::R_WF_FROM, false, A, st);
+        A.src = A.dst;
+        A.dst = c;
+        A.count = ny;
+        fft.cols(plain::C_PLAIN, false, A, st);
     } else if (kind == NADIA_FRESNEL) {
         // FresnelCDI::propagate_from_detector, FresnelCDI.c++:238-243
         plain::multiply_factors(c, coef.p, nx, ny, +1, st);
@@ -927,20 +993,26 @@ void Solver::plain_project(double2 *c)
         plain_scale(padded.p);
         plain_propagate_from(padded.p, true);
         plain::unpad(padded.p, nx, ny, px, py, c, st);
-    } else if (kind == NADIA_PLANAR && nx % 2 == 0 && ny % 2 == 0) {
-        // propagate_to, scale_intensity, propagate_from with the element-wise
-        // steps between the transforms in one kernel (the swap pairs of an
-        // even grid)
-        fft.exec(c, true, st);
-        plain::detector_planar(c, isqrt.p, bs_ptr(), nx, ny, partials.p, d_err.p, st);
+    } else if (kind == NADIA_FRESNEL || (kind == NADIA_PLANAR && nx % 2 == 0 && ny % 2 == 0)) {
+        // the element-wise steps between the two transforms run in the
+        // forward column pass
+        const bool fr = kind == NADIA_FRESNEL;
+        if (fr) plain::invert(c, nx, ny, true, st);
+        plain::Fft64Args A;
+        A.src = A.dst = c;
+        A.s = 1.0 / (sqrt((double)(nx * ny)));
+        A.isqrt = isqrt.p;
+        A.bs = bs_ptr();
+        A.coef = coef.p;
+        A.ill = illum.p;
+        A.swapped = 1;
+        error_args(A, false);
+        A.count = nx;
+        fft.rows(plain::R_PLAIN, true, A, st);
+        A.count = ny;
+        fft.cols(fr ? plain::C_FRESNEL : plain::C_MOD, true, A, st);
         fft.exec(c, false, st);
-    } else if (kind == NADIA_FRESNEL) {
-        plain::invert(c, nx, ny, true, st);
-        fft.exec(c, true, st);
-        plain::detector_fresnel(c, coef.p, illum.p, isqrt.p, bs_ptr(), nx, ny, partials.p,
-                                d_err.p, st);
-        fft.exec(c, false, st);
-        plain::invert(c, nx, ny, true, st);
+        if (fr) plain::invert(c, nx, ny, true, st);
     } else {
         plain_propagate_to(c, false);
         plain_scale(c);
@@ -958,7 +1030,134 @@ void Solver::ensure_temps()
     if (w[PSF] != 0 && !tPSF) tPSF.alloc(n);
 }
 
+double2 *Solver::second()
+{
+    AllocScope scope(st);
+    if (!tPF) tPF.alloc(n);
+    return tPF.p;
+}
+
+// where a pass leaves the error metric; record: in the history as well
+void Solver::error_args(plain::Fft64Args &A, bool record)
+{
+    A.partials = partials.p;
+    A.ticket = ticket.p;
+    A.err = d_err.p;
+    A.ring = record ? d_ring.p : nullptr;
+    A.ring_len = kRing;
+    A.iter = d_iter.p;
+}
+
+// Whether an iteration runs as passes with everything else fused in: even
+// grids, no transmission constraint, and an algorithm whose only projection
+// is Pf x (ER, HIO, RAAR, ...; not the PfPs term).
+bool Solver::fused64() const
+{
+    if ((nx | ny) & 1 || tc.active) return false;
+    if (kind == NADIA_FRESNEL_WF || algorithm == NADIA_ER) return true;
+    return w[PFS] == 0 && w[PF] != 0;
+}
+
+// One iteration.  PlanarCDI and FresnelCDI: rows forward, columns forward with
+// the detector side, rows backward, columns backward with the support and the
+// combine.  PolyCDI: the same on the padded grid, leaving out the rows and
+// columns that are zero or not read, with the expansion in the middle.
+// FresnelCDI_WF: twice the transforms, the swap and the zone-plate factors on
+// the way into the second of each pair.
+void Solver::fused64_iterate()
+{
+    using namespace plain;
+    AllocScope scope(st);
+    const bool er = algorithm == NADIA_ER;
+    Fft64Args A;
+    A.isqrt = isqrt.p;
+    A.bs = bs_ptr();
+    A.sup = support.p;
+    A.coef = coef.p;
+    A.ill = illum.p;
+    A.x = x.p;
+    for (int i = 0; i < 5; ++i) A.w[i] = w[i];
+    A.id = 1 + w[PI];
+    A.er = er;
+    A.use_ps = w[PS] != 0;
+    A.use_psf = w[PSF] != 0;
+    A.wnx = nx;
+    A.wny = ny;
+    error_args(A, true);
+    if (kind == NADIA_POLY) {
+        const int mx = nx + 2 * px, my = ny + 2 * py;
+        A.s = 1.0 / (sqrt((double)(mx * my)));
+        A.px = px;
+        A.py = py;
+        A.src = x.p;
+        A.dst = padded.p + (size_t)px * my; // the transform's row px + i
+        A.count = nx;
+        fft_pad.rows(R_PAD, true, A, st);
+        A.src = A.dst = padded.p;
+        A.q = d_q.p;
+        A.lo = px;
+        A.hi = px + nx;
+        A.count = my;
+        fft_pad.cols(C_POLYQ, true, A, st);
+        poly_gather(d_q.p, d_spec.p, nlambda, d_rows.p, d_cols.p, nx, ny, my, isc.p, st);
+        A.calc = isc.p;
+        A.lo = A.hi = 0;
+        A.count = mx;
+        fft_pad.rows(R_POLY, false, A, st);
+        A.first = py;
+        A.count = ny;
+        fft_pad.cols(C_COMB, false, A, st);
+        return;
+    }
+    A.s = 1.0 / (sqrt((double)(nx * ny)));
+    if (kind == NADIA_FRESNEL_WF) {
+        // FresnelCDI_WF::iterate, FresnelCDI_WF.c++:155-182
+        double2 *t = second();
+        auto rows = [&](RowMode m, bool fwd, const double2 *a, double2 *b) {
+            A.src = a;
+            A.dst = b;
+            A.count = nx;
+            fft.rows(m, fwd, A, st);
+        };
+        auto cols = [&](ColMode m, bool fwd, const double2 *a, double2 *b) {
+            A.src = a;
+            A.dst = b;
+            A.count = ny;
+            fft.cols(m, fwd, A, st);
+        };
+        rows(R_PLAIN, false, x.p, t);
+        cols(C_PLAIN, false, t, t);
+        rows(R_WF_FROM, false, t, x.p);
+        A.er = 1;
+        cols(C_COMB, false, x.p, x.p); // the support, in place
+        rows(R_PLAIN, true, x.p, x.p);
+        cols(C_PLAIN, true, x.p, x.p);
+        rows(R_WF_TO, true, x.p, t);
+        A.s = 1;
+        cols(C_MOD, true, t, x.p);
+        return;
+    }
+    const bool fr = kind == NADIA_FRESNEL;
+    // PlanarCDI's ER needs no copy of x: every pass works in place
+    double2 *P = er && !fr ? x.p : second();
+    A.src = x.p;
+    A.dst = P;
+    A.count = nx;
+    fft.rows(fr ? R_SWAP : R_PLAIN, true, A, st);
+    A.src = P;
+    A.count = ny;
+    A.swapped = 1; // PlanarCDI's detector is centred; FresnelCDI's estimate is
+    fft.cols(fr ? C_FRESNEL : C_MOD, true, A, st);
+    A.count = nx;
+    fft.rows(R_PLAIN, false, A, st);
+    A.count = ny;
+    A.swapped = fr;
+    fft.cols(C_COMB, false, A, st);
+}
+
 // BaseCDI::iterate, BaseCDI.c++:297-387; PolyCDI::iterate, PolyCDI.c++:130-250
+// -- the forms fused64_iterate leaves: odd grids, transmission constraints and
+// algorithms with the PfPs term
 void Solver::plain_iterate_once()
 {
     AllocScope scope(st);
@@ -1018,9 +1217,7 @@ void Solver::plain_iterate_once()
 
 void Solver::record_error()
 {
-    NADIA_CUDA(cudaMemcpyAsync(d_ring.p + (iters % kRing), d_err.p, sizeof(double),
-                               cudaMemcpyDeviceToDevice, st));
-    ++iters;
+    plain::record_error(d_err.p, d_ring.p, kRing, d_iter.p, st);
 }
 
 // BaseCDI::update_n_best, BaseCDI.c++:390-413
@@ -1058,11 +1255,16 @@ void Solver::iterate(int count)
         return;
     }
     for (int it = 0; it < count; ++it) {
-        if (prec == NADIA_FP64)
-            plain_iterate_once();
-        else
+        if (prec == NADIA_FP32) {
             f32->iterate(1);
-        if (prec == NADIA_FP64) record_error();
+        } else if (fused64()) {
+            fused64_iterate();
+            ++iters;
+        } else {
+            plain_iterate_once();
+            record_error();
+            ++iters;
+        }
         if (kind != NADIA_FRESNEL_WF) update_n_best(); // FresnelCDI_WF::iterate keeps none
 
     }

@@ -47,6 +47,8 @@ struct Solver {
     DevBuf<double> d_err;     // [0] current error
     DevBuf<double> d_ring;    // kRing errors
     DevBuf<double> partials;  // reduction scratch
+    DevBuf<long long> d_iter; // FP64: iterations recorded in d_ring
+    DevBuf<unsigned> ticket;  // FP64: blocks of a pass that have left their error sums
 
     // n-best (BaseCDI.c++:43-50, 390-413): slot buffers, rank order, errors
     std::vector<DevBuf<double2>> best64;
@@ -77,6 +79,8 @@ struct Solver {
     bool has_spectrum = false;
     DevBuf<double> d_spec, isc;
     DevBuf<double2> padded;
+    DevBuf<double> d_q;           // |Psi|^2 of the centred padded field
+    DevBuf<int> d_rows, d_cols;   // sample rows (as offsets) and columns of each line
     plain::Fft2d fft_pad;
 
     // TransmissionConstraint set by BaseCDI::set_complex_constraint (FP64 form)
@@ -144,6 +148,13 @@ struct Solver {
 
     // FP64 plain path internals
     void plain_iterate_once();
+    bool fused64() const;
+    void fused64_iterate();
+    void error_args(plain::Fft64Args &A, bool record);
+    double2 *second(); // a second estimate-sized buffer (also the combine's Pf term)
+    void plain_partials(size_t blocks);
+    void poly_tables();
+    void plain_counters();
     void plain_project(double2 *c);
     void plain_propagate_to(double2 *c, bool padded_grid);
     void plain_propagate_from(double2 *c, bool padded_grid);
