@@ -918,89 +918,105 @@ void Fused32::Impl::prepare_pfs()
     if (!pfs_choice) pfs_choice = &choose(nx, ny, S.kind == NADIA_FRESNEL, 1, true);
 }
 
-// Host arrays are in the reference's order (element (x, y) at x*ny + y); the
-// device arrays in the panel layout.  The host converts, so uploads and
-// readbacks are plain copies: they run on the copy engines and never wait
-// for SMs held by other reconstructions' passes.
-namespace {
-// host array (x*ny + y order, stride values per element, of type T) to the
-// panel layout in FP32, converted in the same pass
-template <class T>
-void to_panel(const T *h, int stride, float *p, int nx, int ny, bool fold)
+// Rows r0 .. r0+rows-1 of an array in the reference's order (element (x, y) at
+// x*ny + y), in mapped host memory, to or from the panel layout.  A thread
+// moves 16 bytes: STRIDE neighbouring ones are four columns of a panel row.
+// The host side of the transfer crosses the link as full warps' runs of 512
+// bytes, so the order costs no pass of its own on either side.  `fold` moves
+// PlanarCDI's centred detector to transform order.
+template <int STRIDE>
+__global__ void k_panel_put(const float4 *__restrict__ h, float4 *__restrict__ d, int nx, int ny,
+                            int r0, int rows, int fold)
 {
-    // x outer, y inner: the source is read in order, and the panel rows a
-    // column writes (16 bytes each) are the next column's neighbours
-    for (int kx = 0; kx < nx; ++kx) {
-        int dx = kx;
-        if (fold) {
-            dx = kx + nx / 2;
-            dx = dx >= nx ? dx - nx : dx;
+    const int q = ny / kPanel * STRIDE; // 16-byte units of a row
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < rows * q; e += gridDim.x * blockDim.x) {
+        int x = r0 + e / q;
+        const int f = e % q, half = f % STRIDE;
+        int p = f / STRIDE;
+        if (fold) { // source (dx, dy) belongs at (dx + nx/2, dy + ny/2)
+            x += nx / 2;
+            x = x >= nx ? x - nx : x;
+            p += ny / kPanel / 2;
+            p = p >= ny / kPanel ? p - ny / kPanel : p;
         }
-        const T *src = h + (size_t)dx * ny * stride;
-        for (int ky = 0; ky < ny; ++ky) {
-            int dy = ky;
-            if (fold) {
-                dy = ky + ny / 2;
-                dy = dy >= ny ? dy - ny : dy;
-            }
-            const size_t a = panel_index_dev(kx, ky, nx);
-            for (int c = 0; c < stride; ++c) p[a * stride + c] = (float)src[(size_t)dy * stride + c];
-        }
+        d[((size_t)p * nx + x) * STRIDE + half] = __ldcs(&h[e]);
     }
+}
+
+template <int STRIDE>
+__global__ void k_panel_get(const float4 *__restrict__ d, float4 *__restrict__ h, int nx, int ny,
+                            int r0, int rows)
+{
+    const int q = ny / kPanel * STRIDE;
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < rows * q; e += gridDim.x * blockDim.x) {
+        const int x = r0 + e / q, f = e % q, p = f / STRIDE, half = f % STRIDE;
+        __stcs(&h[e], d[((size_t)p * nx + x) * STRIDE + half]);
+    }
+}
+
+namespace {
+// blocks of a piece's reordering kernel: enough to fill the link, few enough
+// to leave the GPU to other reconstructions' passes
+constexpr int kPanelBlocks = 64, kPanelThreads = 512;
+
+template <class T>
+void put_rows(const T *h, int stride, void *dst, bool fold, int nx, int ny, int device,
+              cudaStream_t st)
+{
+    const size_t w = (size_t)ny * stride;
+    in_pieces(device, nx, w * sizeof(float), [&](CopySlot &slot, size_t r0, size_t rows) {
+        float *p = static_cast<float *>(slot.p);
+        const T *src = h + r0 * w;
+        for (size_t k = 0; k < rows * w; ++k) p[k] = (float)src[k];
+        if (stride == 1)
+            k_panel_put<1><<<kPanelBlocks, kPanelThreads, 0, st>>>(
+                (const float4 *)p, (float4 *)dst, nx, ny, (int)r0, (int)rows, fold);
+        else
+            k_panel_put<2><<<kPanelBlocks, kPanelThreads, 0, st>>>(
+                (const float4 *)p, (float4 *)dst, nx, ny, (int)r0, (int)rows, fold);
+        NADIA_CUDA(cudaGetLastError());
+        slot.wait(st);
+    });
+}
+
+template <class T>
+void get_rows(const void *src, int stride, T *h, int nx, int ny, int device, cudaStream_t st)
+{
+    const size_t w = (size_t)ny * stride;
+    in_pieces(device, nx, w * sizeof(float), [&](CopySlot &slot, size_t r0, size_t rows) {
+        const float *p = static_cast<const float *>(slot.p);
+        if (stride == 1)
+            k_panel_get<1><<<kPanelBlocks, kPanelThreads, 0, st>>>(
+                (const float4 *)src, (float4 *)slot.p, nx, ny, (int)r0, (int)rows);
+        else
+            k_panel_get<2><<<kPanelBlocks, kPanelThreads, 0, st>>>(
+                (const float4 *)src, (float4 *)slot.p, nx, ny, (int)r0, (int)rows);
+        NADIA_CUDA(cudaGetLastError());
+        slot.wait(st);
+        T *dst = h + r0 * w;
+        for (size_t k = 0; k < rows * w; ++k) dst[k] = (T)p[k];
+    });
 }
 } // namespace
 
-// the host staging array of the conversions, kept between calls (a fresh
-// one would be page-faulted in again on every upload and readback)
-float *Fused32::Impl::staging(size_t count)
-{
-    if (stage.size() < count) stage.resize(count);
-    return stage.data();
-}
-
 void Fused32::Impl::put_panel_f(const float *h, int stride, void *dst, bool fold)
 {
-    float *p = staging(n * stride);
-    to_panel(h, stride, p, nx, ny, fold);
-    NADIA_CUDA(cudaMemcpyAsync(dst, p, n * stride * sizeof(float), cudaMemcpyHostToDevice, S.st));
-    NADIA_CUDA(cudaStreamSynchronize(S.st));
+    put_rows(h, stride, dst, fold, nx, ny, S.device, S.st);
 }
 
 void Fused32::Impl::put_panel(const double *h, int stride, void *dst, bool fold)
 {
-    float *p = staging(n * stride);
-    to_panel(h, stride, p, nx, ny, fold);
-    NADIA_CUDA(cudaMemcpyAsync(dst, p, n * stride * sizeof(float), cudaMemcpyHostToDevice, S.st));
-    NADIA_CUDA(cudaStreamSynchronize(S.st));
+    put_rows(h, stride, dst, fold, nx, ny, S.device, S.st);
 }
-
-namespace {
-// panel layout (FP32) to the reference's order, converted to T in the pass
-template <class T>
-void from_panel(const float *p, int stride, T *h, int nx, int ny)
-{
-    for (int xx = 0; xx < nx; ++xx)
-        for (int yy = 0; yy < ny; ++yy) {
-            const size_t a = panel_index_dev(xx, yy, nx), d = (size_t)xx * ny + yy;
-            for (int c = 0; c < stride; ++c) h[d * stride + c] = (T)p[a * stride + c];
-        }
-}
-} // namespace
 
 void Fused32::Impl::get_panel_f(const void *src, int stride, float *h)
 {
-    float *p = staging(n * stride);
-    NADIA_CUDA(cudaMemcpyAsync(p, src, n * stride * sizeof(float), cudaMemcpyDeviceToHost, S.st));
-    NADIA_CUDA(cudaStreamSynchronize(S.st));
-    from_panel(p, stride, h, nx, ny);
+    get_rows(src, stride, h, nx, ny, S.device, S.st);
 }
 
 void Fused32::Impl::get_panel(const void *src, int stride, double *h)
 {
-    float *p = staging(n * stride);
-    NADIA_CUDA(cudaMemcpyAsync(p, src, n * stride * sizeof(float), cudaMemcpyDeviceToHost, S.st));
-    NADIA_CUDA(cudaStreamSynchronize(S.st));
-    from_panel(p, stride, h, nx, ny);
+    get_rows(src, stride, h, nx, ny, S.device, S.st);
 }
 
 // set_intensity and set_beam_stop mark sqrt(I) for conversion; it is formed

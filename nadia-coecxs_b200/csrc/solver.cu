@@ -34,15 +34,19 @@ void retain_pool_memory()
 }
 
 namespace {
+int current_device()
+{
+    int dev = 0;
+    NADIA_CUDA(cudaGetDevice(&dev));
+    return dev;
+}
 void h2d(void *d, const void *h, size_t bytes, cudaStream_t s)
 {
-    NADIA_CUDA(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, s));
-    NADIA_CUDA(cudaStreamSynchronize(s));
+    to_device(d, h, bytes, current_device(), s);
 }
 void d2h(void *h, const void *d, size_t bytes, cudaStream_t s)
 {
-    NADIA_CUDA(cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, s));
-    NADIA_CUDA(cudaStreamSynchronize(s));
+    to_host(h, d, bytes, current_device(), s);
 }
 // The C library's srand(seed)/rand() sequence (the reference seeds and draws
 // with them in initialise_estimate) from a private generator state: glibc's
@@ -1285,9 +1289,10 @@ void Solver::get_error_history(double *out, int count)
     AllocScope scope(st);
     NADIA_REQUIRE(count >= 0 && count <= kRing && count <= iters, NADIA_ERR_RANGE,
                   "fewer iterations recorded than requested");
-    std::vector<double> ring(kRing);
-    d2h(ring.data(), d_ring.p, d_ring.bytes(), st);
-    for (int i = 0; i < count; ++i) out[i] = ring[(size_t)((iters - count + i) % kRing)];
+    // the last `count` slots of the ring: at most two runs
+    const int first = (int)((iters - count) % kRing), run = std::min(count, kRing - first);
+    if (run > 0) d2h(out, d_ring.p + first, run * sizeof(double), st);
+    if (count > run) d2h(out + run, d_ring.p, (count - run) * sizeof(double), st);
 }
 
 // BaseCDI::apply_shrinkwrap, BaseCDI.c++:416-429

@@ -10,6 +10,7 @@
 
 #include "common.h"
 #include "plain64.h"
+#include "transfer.h"
 
 namespace nadia {
 
@@ -26,6 +27,7 @@ struct Solver {
     // bumped whenever the support or the Fresnel illumination changes (the
     // inputs of a phase-diverse object's weights)
     unsigned long long weights_version = 0;
+    PinnedSlots::User slots;
     OwnedStream own_st;         // outlives every buffer below
     cudaStream_t st = nullptr;
 

@@ -1,0 +1,113 @@
+// transfer.cu -- pinned slots, the copying threads' budget and plain copies.
+#include "transfer.h"
+
+#include <cstring>
+#include <vector>
+
+namespace nadia {
+
+namespace {
+// leaked on purpose: reconstructions destroyed by static destructors still use them
+std::mutex &slot_mu()
+{
+    static std::mutex *m = new std::mutex;
+    return *m;
+}
+std::vector<void *> &free_slots()
+{
+    static std::vector<void *> *v = new std::vector<void *>;
+    return *v;
+}
+size_t g_users = 0;
+std::atomic<int> g_threads{0};
+} // namespace
+
+PinnedSlots::User::User()
+{
+    std::lock_guard<std::mutex> lk(slot_mu());
+    ++g_users;
+}
+
+PinnedSlots::User::~User()
+{
+    std::lock_guard<std::mutex> lk(slot_mu());
+    if (--g_users > 0) return;
+    for (void *p : free_slots()) cudaFreeHost(p);
+    free_slots().clear();
+}
+
+void *PinnedSlots::take()
+{
+    {
+        std::lock_guard<std::mutex> lk(slot_mu());
+        if (!free_slots().empty()) {
+            void *p = free_slots().back();
+            free_slots().pop_back();
+            return p;
+        }
+    }
+    void *p = nullptr;
+    NADIA_CUDA(cudaHostAlloc(&p, kSlotBytes, cudaHostAllocPortable | cudaHostAllocMapped));
+    return p;
+}
+
+void PinnedSlots::give(void *p)
+{
+    {
+        std::lock_guard<std::mutex> lk(slot_mu());
+        if (g_users > 0 && free_slots().size() < kKeep) {
+            free_slots().push_back(p);
+            return;
+        }
+    }
+    cudaFreeHost(p);
+}
+
+int borrow_threads(int wanted)
+{
+    static const int all = std::max(0, (int)std::thread::hardware_concurrency() / 2);
+    int have = g_threads.load();
+    for (;;) {
+        const int n = std::max(0, std::min(wanted, all - have));
+        if (g_threads.compare_exchange_weak(have, have + n)) return n;
+    }
+}
+
+void return_threads(int n) { g_threads -= n; }
+
+namespace {
+constexpr size_t kRow = 64 << 10;      // plain copies are cut in "rows" of this size
+constexpr size_t kSmallCopy = 2 << 20; // below: the driver's own staging (about 16 GB/s)
+} // namespace
+
+void to_device(void *d, const void *h, size_t bytes, int device, cudaStream_t st)
+{
+    if (bytes < kSmallCopy) {
+        NADIA_CUDA(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, st));
+        NADIA_CUDA(cudaStreamSynchronize(st));
+        return;
+    }
+    in_pieces(device, (bytes + kRow - 1) / kRow, kRow, [&](CopySlot &slot, size_t r, size_t rows) {
+        const size_t at = r * kRow, len = std::min(rows * kRow, bytes - at);
+        std::memcpy(slot.p, (const char *)h + at, len);
+        NADIA_CUDA(cudaMemcpyAsync((char *)d + at, slot.p, len, cudaMemcpyHostToDevice, st));
+        slot.wait(st);
+    });
+}
+
+void to_host(void *h, const void *d, size_t bytes, int device, cudaStream_t st)
+{
+    if (bytes < kSmallCopy) {
+        NADIA_CUDA(cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, st));
+        NADIA_CUDA(cudaStreamSynchronize(st));
+        return;
+    }
+    in_pieces(device, (bytes + kRow - 1) / kRow, kRow, [&](CopySlot &slot, size_t r, size_t rows) {
+        const size_t at = r * kRow, len = std::min(rows * kRow, bytes - at);
+        NADIA_CUDA(cudaMemcpyAsync(slot.p, (const char *)d + at, len, cudaMemcpyDeviceToHost, st));
+        slot.wait(st);
+        std::memcpy((char *)h + at, slot.p, len);
+    });
+}
+
+} // namespace nadia

@@ -1,0 +1,124 @@
+// transfer.h -- arrays between host memory and the device.
+//
+// A caller's arrays are pageable: a copy straight from or to them runs through
+// the driver's single staging thread, and a freshly allocated result is
+// page-faulted in by that same thread (a 2048^2 complex128 estimate: 14.3 ms,
+// 4.7 GB/s on B200 over a link that carries ten times that).  Here an array is
+// cut into pieces of whole rows; several threads take piece after piece, each
+// through a pinned slot of its own, so one piece's conversion and page faults
+// run beside the others' transfers.
+#pragma once
+
+#include <algorithm>
+#include <exception>
+#include <mutex>
+#include <system_error>
+#include <thread>
+
+#include "common.h"
+
+namespace nadia {
+
+constexpr size_t kSlotBytes = 4u << 20; // one pinned slot
+
+// Pinned slots of the process: at most kKeep unused ones are kept, and none
+// once the last reconstruction is gone.
+class PinnedSlots {
+public:
+    // held by every reconstruction
+    struct User {
+        User();
+        ~User();
+        User(const User &) = delete;
+        User &operator=(const User &) = delete;
+    };
+    static void *take();
+    static void give(void *p);
+
+private:
+    static constexpr size_t kKeep = 16;
+};
+
+// threads that copies of this process may use now beside their callers:
+// half the cores between all concurrent copies
+int borrow_threads(int wanted);
+void return_threads(int n);
+
+struct CopySlot {
+    void *p = nullptr;
+    cudaEvent_t ev = nullptr;
+    CopySlot()
+    {
+        p = PinnedSlots::take();
+        const cudaError_t e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+        if (e != cudaSuccess) {
+            PinnedSlots::give(p);
+            NADIA_CUDA(e);
+        }
+    }
+    ~CopySlot()
+    {
+        cudaEventSynchronize(ev); // work queued on the slot before an error
+        cudaEventDestroy(ev);
+        PinnedSlots::give(p);
+    }
+    CopySlot(const CopySlot &) = delete;
+    CopySlot &operator=(const CopySlot &) = delete;
+    // waits until what was queued on st by now is done
+    void wait(cudaStream_t st)
+    {
+        NADIA_CUDA(cudaEventRecord(ev, st));
+        NADIA_CUDA(cudaEventSynchronize(ev));
+    }
+};
+
+// Calls body(slot, first row, rows) for pieces of `rows` rows of `row_bytes`
+// (as they pass through a slot); each piece is done when its call returns.
+// The first error of any thread is thrown once all have stopped.
+template <class Body>
+void in_pieces(int device, size_t rows, size_t row_bytes, Body body)
+{
+    NADIA_REQUIRE(row_bytes <= kSlotBytes, NADIA_ERR_INVALID, "row too long to transfer");
+    if (rows == 0) return;
+    const size_t fit = kSlotBytes / row_bytes;
+    // two pieces a thread at least, and pieces worth a thread's start
+    const size_t worth = std::max<size_t>(1, (1u << 20) / row_bytes);
+    const int most = (int)std::min<size_t>(8, rows / worth + 1);
+    const int extra = borrow_threads(most - 1);
+    const size_t per = std::max<size_t>(1, std::min(fit, (rows + 2 * (extra + 1) - 1) / (2 * (extra + 1))));
+    std::atomic<size_t> next{0};
+    std::exception_ptr error;
+    std::mutex mu;
+    auto work = [&](bool own) {
+        try {
+            if (!own) NADIA_CUDA(cudaSetDevice(device));
+            CopySlot slot;
+            for (;;) {
+                const size_t r = next.fetch_add(per);
+                if (r >= rows) break;
+                body(slot, r, std::min(per, rows - r));
+            }
+        } catch (...) {
+            next = rows;
+            std::lock_guard<std::mutex> lk(mu);
+            if (!error) error = std::current_exception();
+        }
+    };
+    std::thread pool[8];
+    int started = 0;
+    try {
+        for (; started < extra; ++started) pool[started] = std::thread(work, false);
+    } catch (const std::system_error &) {
+        // fewer threads then
+    }
+    work(true);
+    for (int i = 0; i < started; ++i) pool[i].join();
+    return_threads(extra);
+    if (error) std::rethrow_exception(error);
+}
+
+// Copies that are complete when they return, ordered after the work queued on st.
+void to_device(void *d, const void *h, size_t bytes, int device, cudaStream_t st);
+void to_host(void *h, const void *d, size_t bytes, int device, cudaStream_t st);
+
+} // namespace nadia
