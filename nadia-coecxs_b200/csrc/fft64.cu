@@ -19,10 +19,10 @@ NADIA_P2(2048)
 NADIA_P2(4096)
 #undef NADIA_P2
 #define NADIA_ANY(L)                                                                             \
-    void rows_any##L(RowMode mode, bool fwd, const Fft64Args &A, const Fft64Plan &p, size_t smem, \
-                     cudaStream_t st);                                                           \
-    void cols_any##L(ColMode mode, bool fwd, const Fft64Args &A, const Fft64Plan &p, size_t smem, \
-                     cudaStream_t st);
+    void rows_any##L(RowMode mode, bool fwd, const Fft64Args &A, const Fft64Plan &p, int threads, \
+                     size_t smem, cudaStream_t st);                                                           \
+    void cols_any##L(ColMode mode, bool fwd, const Fft64Args &A, const Fft64Plan &p, int threads, \
+                     size_t smem, cudaStream_t st);
 NADIA_ANY(1)
 NADIA_ANY(2)
 NADIA_ANY(4)
@@ -58,15 +58,17 @@ bool launch_cols_p2(int N, int L, ColMode mode, bool fwd, const Fft64Args &A, cu
 }
 
 void launch_rows_any(int L, RowMode mode, bool fwd, const Fft64Args &A, const Fft64Plan &p,
-                     size_t smem, cudaStream_t st)
+                     int threads, size_t smem, cudaStream_t st)
 {
-    (L == 1 ? rows_any1 : L == 2 ? rows_any2 : L == 4 ? rows_any4 : rows_any8)(mode, fwd, A, p, smem, st);
+    (L == 1 ? rows_any1 : L == 2 ? rows_any2 : L == 4 ? rows_any4 : rows_any8)(
+        mode, fwd, A, p, threads, smem, st);
 }
 
 void launch_cols_any(int L, ColMode mode, bool fwd, const Fft64Args &A, const Fft64Plan &p,
-                     size_t smem, cudaStream_t st)
+                     int threads, size_t smem, cudaStream_t st)
 {
-    (L == 1 ? cols_any1 : L == 2 ? cols_any2 : L == 4 ? cols_any4 : cols_any8)(mode, fwd, A, p, smem, st);
+    (L == 1 ? cols_any1 : L == 2 ? cols_any2 : L == 4 ? cols_any4 : cols_any8)(
+        mode, fwd, A, p, threads, smem, st);
 }
 
 namespace {
@@ -75,8 +77,7 @@ constexpr size_t kSmemMax = 227 * 1024;
 // two neighbouring radices whose passes one thread can do on its registers
 bool joinable(int a, int b)
 {
-    return (a == 8 && b == 2) || (a == 4 && b == 3) || (a == 2 && (b == 3 || b == 5)) ||
-           (a == 3 && (b == 3 || b == 5));
+    return (a == 2 && (b == 3 || b == 5)) || (a == 3 && b == 3);
 }
 } // namespace
 
@@ -153,12 +154,42 @@ int Fft64Axis::tile_p2(int count, bool cols) const
     return L;
 }
 
-int Fft64Axis::tile_any(int count, bool cols) const
+// Signals and threads to a block of the any-length kernels: the pair with the
+// least estimated time for `count` signals.  A block's time is a latency per
+// pass and round (a barrier and a trip through shared memory) plus the rounds'
+// work; an SM runs as many blocks as its registers and shared memory hold.
+void Fft64Axis::shape_any(int count, bool cols, int *Lout, int *threads) const
 {
-    int L = 8;
-    const int least = cols && smem_any(2) <= kSmemMax ? 2 : 1;
-    while (L > least && (smem_any(L) > 72 * 1024 || (count + L - 1) / L < 296)) L /= 2;
-    return L;
+    double best = 1e300;
+    for (int L = 1; L <= 8; L *= 2) {
+        const size_t smem = smem_any(L);
+        if (smem > kSmemMax) break;
+        if (cols && L == 1 && smem_any(2) <= kSmemMax) continue; // half-used sectors
+        for (int nt = 64; nt <= kAnyMaxThreads; nt += 32) {
+            const int tiles = (count + L - 1) / L;
+            int held = std::min({65536 / (kAnyRegisters * nt), (int)(kSmemMax / (smem + 1024)), 32});
+            held = std::max(1, std::min(held, (tiles + 147) / 148));
+            const int waves = (tiles + 148 * held - 1) / (148 * held);
+            double t = 2000 + 2.0 * ((L * plan.n + nt - 1) / nt) * 40; // load and store
+            double work = 0; // issue slots of the block's warps
+            for (int i = 0; i < plan.np; ++i) {
+                const int R = plan.pass[i].r1 * plan.pass[i].r2, m = plan.n / R;
+                const bool prime = plan.pass[i].r1 > 8;
+                const int items = prime ? (R + 3) / 4 * L * m : L * m;
+                const int rounds = (items + nt - 1) / nt;
+                const double each = prime ? R * 70.0 : R * 25.0; // cycles of one item
+                t += 400 + rounds * (200 + each);
+                work += rounds * (nt / 32) * (prime ? R * 64.0 : R * 30.0);
+            }
+            // four schedulers share the work of the blocks an SM holds
+            const double time = waves * std::max(t, held * work / 4);
+            if (time < best) {
+                best = time;
+                *Lout = L;
+                *threads = nt;
+            }
+        }
+    }
 }
 
 void Fft2d::init(int nx_, int ny_)
@@ -169,30 +200,36 @@ void Fft2d::init(int nx_, int ny_)
     Y.init(ny);
 }
 
-void Fft2d::rows(RowMode mode, bool forward, Fft64Args A, cudaStream_t s) const
+int Fft2d::rows(RowMode mode, bool forward, Fft64Args A, cudaStream_t s) const
 {
     A.nx = nx;
     A.ny = ny;
     A.tw = Y.tw.p;
-    if (!(Y.p2 && launch_rows_p2(ny, Y.tile_p2(A.count, false), mode, forward, A, s))) {
-        const int L = Y.tile_any(A.count, false);
-        launch_rows_any(L, mode, forward, A, Y.plan, Y.smem_any(L), s);
+    int L = Y.p2 ? Y.tile_p2(A.count, false) : 0;
+    if (!(L && launch_rows_p2(ny, L, mode, forward, A, s))) {
+        int nt;
+        Y.shape_any(A.count, false, &L, &nt);
+        launch_rows_any(L, mode, forward, A, Y.plan, nt, Y.smem_any(L), s);
     }
     NADIA_CUDA(cudaGetLastError());
+    return (A.count + L - 1) / L;
 }
 
-void Fft2d::cols(ColMode mode, bool forward, Fft64Args A, cudaStream_t s) const
+int Fft2d::cols(ColMode mode, bool forward, Fft64Args A, cudaStream_t s) const
 {
     A.nx = nx;
     A.ny = ny;
     A.tw = X.tw.p;
     if (A.hi == 0) A.hi = nx;
     const bool whole = A.lo == 0 && A.hi == nx;
-    if (!(X.p2 && whole && launch_cols_p2(nx, X.tile_p2(A.count, true), mode, forward, A, s))) {
-        const int L = X.tile_any(A.count, true);
-        launch_cols_any(L, mode, forward, A, X.plan, X.smem_any(L), s);
+    int L = X.p2 && whole ? X.tile_p2(A.count, true) : 0;
+    if (!(L && launch_cols_p2(nx, L, mode, forward, A, s))) {
+        int nt;
+        X.shape_any(A.count, true, &L, &nt);
+        launch_cols_any(L, mode, forward, A, X.plan, nt, X.smem_any(L), s);
     }
     NADIA_CUDA(cudaGetLastError());
+    return (A.count + L - 1) / L;
 }
 
 void Fft2d::exec(double2 *a, bool forward, cudaStream_t s) const

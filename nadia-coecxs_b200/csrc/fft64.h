@@ -56,6 +56,9 @@ struct Fft64Pass {
     FastDiv dNs, dm;                     // division by Ns and by n / (r1 * r2)
 };
 
+// the any-length kernels' launch bounds
+constexpr int kAnyMaxThreads = 256, kAnyRegisters = 80;
+
 constexpr int kMaxSuper = 14;
 struct Fft64Plan {
     int n, np, swz; // swz: the first pass's power of two (bank swizzle), 0 for odd
@@ -87,10 +90,12 @@ struct Fft64Args {
     int wnx = 0, wny = 0, px = 0, py = 0; // PolyCDI: the unpadded grid and its offset
     const double *calc = nullptr;         // PolyCDI: sqrt of the expanded intensity
     double *q = nullptr;
-    // error metric: one partial pair per block, summed by the last block to
-    // finish (in block order) into *err and ring[*iter % ring_len]
+    // error metric: a pass with a modulus leaves one pair of sums per block in
+    // `partials`; the next pass, given their number in `pairs`, has one block
+    // more than its tiles, which adds them up into *err and
+    // ring[*iter % ring_len] beside the transforms
     double *partials = nullptr, *err = nullptr, *ring = nullptr;
-    unsigned *ticket = nullptr;
+    int pairs = 0;
     long long *iter = nullptr;
     int ring_len = 1;
 };
@@ -103,9 +108,8 @@ struct Fft64Axis {
     bool p2 = false; // 64 ... 4096, a power of two
     int max_prime = 0;
     void init(int n);
-    // signals to a block: p2 and any-length kernels
-    int tile_p2(int count, bool cols) const;
-    int tile_any(int count, bool cols) const;
+    int tile_p2(int count, bool cols) const; // signals to a block
+    void shape_any(int count, bool cols, int *L, int *threads) const;
     size_t smem_any(int L) const;
 };
 
@@ -114,9 +118,9 @@ bool launch_rows_p2(int N, int L, RowMode mode, bool fwd, const Fft64Args &A, cu
 bool launch_cols_p2(int N, int L, ColMode mode, bool fwd, const Fft64Args &A, cudaStream_t st);
 // fft64_any*.cu
 void launch_rows_any(int L, RowMode mode, bool fwd, const Fft64Args &A, const Fft64Plan &p,
-                     size_t smem, cudaStream_t st);
+                     int threads, size_t smem, cudaStream_t st);
 void launch_cols_any(int L, ColMode mode, bool fwd, const Fft64Args &A, const Fft64Plan &p,
-                     size_t smem, cudaStream_t st);
+                     int threads, size_t smem, cudaStream_t st);
 
 // In-place unnormalised 2-D DFT of an nx-by-ny row-major double2 array with
 // the canonical Stockham schedule: every row (length ny), then every column.
@@ -125,10 +129,33 @@ struct Fft2d {
     Fft64Axis X, Y; // columns (length nx), rows (length ny)
     void init(int nx, int ny);
     void exec(double2 *a, bool forward, cudaStream_t s) const;
-    // rows/columns A.first .. +A.count-1 in a fused mode; nx, ny and tw are filled in
-    void rows(RowMode mode, bool forward, Fft64Args A, cudaStream_t s) const;
-    void cols(ColMode mode, bool forward, Fft64Args A, cudaStream_t s) const;
+    // rows/columns A.first .. +A.count-1 in a fused mode; nx, ny and tw are
+    // filled in.  Returns the number of blocks (pairs of error sums).
+    int rows(RowMode mode, bool forward, Fft64Args A, cudaStream_t s) const;
+    int cols(ColMode mode, bool forward, Fft64Args A, cudaStream_t s) const;
 };
+
+// the error metric from `pairs` pairs of sums, where no pass follows
+void finish_error(const Fft64Args &A, cudaStream_t s);
+
+// launches a pass so that it may start while the work before it on st drains
+// (the kernel waits for it, see after_previous)
+template <class... P, class... V>
+void launch_pass(void (*kernel)(P...), int blocks, int threads, size_t smem, cudaStream_t st,
+                 const V &...args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    NADIA_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+}
 
 // the largest dynamic shared memory a kernel may have, raised once per device
 template <class K>

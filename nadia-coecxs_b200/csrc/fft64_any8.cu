@@ -4,16 +4,16 @@
 namespace nadia {
 namespace plain {
 
-void rows_any8(RowMode mode, bool fwd, const Fft64Args &A, const Fft64Plan &p, size_t smem,
-               cudaStream_t st)
+void rows_any8(RowMode mode, bool fwd, const Fft64Args &A, const Fft64Plan &p,
+               int threads, size_t smem, cudaStream_t st)
 {
-    rows_any_modes<8>(mode, fwd, A, p, smem, st);
+    rows_any_modes<8>(mode, fwd, A, p, threads, smem, st);
 }
 
-void cols_any8(ColMode mode, bool fwd, const Fft64Args &A, const Fft64Plan &p, size_t smem,
-               cudaStream_t st)
+void cols_any8(ColMode mode, bool fwd, const Fft64Args &A, const Fft64Plan &p,
+               int threads, size_t smem, cudaStream_t st)
 {
-    cols_any_modes<8>(mode, fwd, A, p, smem, st);
+    cols_any_modes<8>(mode, fwd, A, p, threads, smem, st);
 }
 
 } // namespace plain

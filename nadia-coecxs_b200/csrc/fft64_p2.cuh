@@ -16,16 +16,19 @@ namespace nadia {
 namespace plain {
 namespace {
 
-// The passes of a length: 8s, then the remaining 4, or the remaining 2 joined
-// to the last 8 (sixteen values a thread).
+// The passes of a length: 8s, then the remaining 4 or 2.  At 1024 points the 2 is
+// joined to the last 8 (sixteen values a thread, one exchange less: HIO 1024^2
+// 53.3 us against 56.3); at 128 points the grid is too small for half as many
+// threads (128^2 23 us joined, 15.5 not).
 template <int N>
 struct P2 {
     static constexpr int lg = N <= 64 ? 6 : N <= 128 ? 7 : N <= 256 ? 8 : N <= 512 ? 9
                             : N <= 1024 ? 10 : N <= 2048 ? 11 : 12;
-    static constexpr int np = lg / 3 + (lg % 3 == 2);
-    static constexpr int EPT = lg % 3 == 1 ? 16 : 8;
-    static constexpr int r1(int p) { return p < lg / 3 ? 8 : 4; }
-    static constexpr int r2(int p) { return lg % 3 == 1 && p == np - 1 ? 2 : 1; }
+    static constexpr bool join = lg == 10;
+    static constexpr int np = lg / 3 + (lg % 3 != 0 && !join);
+    static constexpr int EPT = join ? 16 : 8;
+    static constexpr int r1(int p) { return p < lg / 3 ? 8 : lg % 3 == 2 ? 4 : 2; }
+    static constexpr int r2(int p) { return join && p == np - 1 ? 2 : 1; }
     static constexpr int span(int p) { return p == 0 ? 1 : span(p - 1) * r1(p - 1) * r2(p - 1); }
     static constexpr int tw(int p) // offset of the pass's twiddles: the first pass has none
     {
@@ -58,6 +61,7 @@ __device__ __forceinline__ void passes(double2 *v, double2 *sm, const double2 *_
         super<R1, R2, FWD>(v + q * R, P == 0 ? 0 : j % Ns, Ns, t1, t2, nullptr, nullptr);
     }
     if constexpr (P == PL::np - 1) {
+        let_next_start();
 #pragma unroll
         for (int q = 0; q < NB; ++q) {
             const int b = threadIdx.x + q * NT, sig = b % L, j = b / L;
@@ -101,8 +105,13 @@ template <int N, int L, int MODE, bool FWD>
 __global__ void __launch_bounds__(Tile64<N, L>::nt, Tile64<N, L>::minb) k_rows_p2(const Fft64Args A)
 {
     extern __shared__ double2 sm[];
+    after_previous();
     constexpr int NT = Tile64<N, L>::nt, R = P2<N>::r1(0), NB = P2<N>::EPT / R, m = N / R;
     const int r0 = A.first + blockIdx.x * L, end = A.first + A.count;
+    if (A.pairs && r0 >= end) {
+        add_errors(A, sm);
+        return;
+    }
     double2 v[P2<N>::EPT];
     double diff = 0, mag = 0;
 #pragma unroll
@@ -129,8 +138,13 @@ template <int N, int L, int MODE, bool FWD>
 __global__ void __launch_bounds__(Tile64<N, L>::nt, Tile64<N, L>::minb) k_cols_p2(const Fft64Args A)
 {
     extern __shared__ double2 sm[];
+    after_previous();
     constexpr int NT = Tile64<N, L>::nt, R = P2<N>::r1(0), NB = P2<N>::EPT / R, m = N / R;
     const int c0 = A.first + blockIdx.x * L, end = A.first + A.count;
+    if (A.pairs && c0 >= end) {
+        add_errors(A, sm);
+        return;
+    }
     double2 v[P2<N>::EPT];
     double diff = 0, mag = 0;
 #pragma unroll
@@ -142,7 +156,7 @@ __global__ void __launch_bounds__(Tile64<N, L>::nt, Tile64<N, L>::minb) k_cols_p
     }
     passes<N, L, NT, FWD, 0>(v, sm, A.tw, [&](int sig, int base, const double2 *o) {
         constexpr int P = P2<N>::np - 1, R1 = P2<N>::r1(P), R2 = P2<N>::r2(P), Ns = P2<N>::span(P);
-        constexpr int R_ = R1 * R2, G = 4;
+        constexpr int R_ = R1 * R2, G = R_ < 4 ? R_ : 4;
         const int c = c0 + sig;
         if (c < end) {
 #pragma unroll
@@ -158,7 +172,7 @@ __global__ void __launch_bounds__(Tile64<N, L>::nt, Tile64<N, L>::minb) k_cols_p
             }
         }
     });
-    if constexpr (MODE == C_MOD || MODE == C_FRESNEL) finish_error(A, diff, mag, sm);
+    if constexpr (MODE == C_MOD || MODE == C_FRESNEL) leave_error(A, diff, mag, sm);
 }
 
 template <int N, int L, int MODE, bool FWD>
@@ -166,7 +180,8 @@ void rows_p2(const Fft64Args &A, cudaStream_t st)
 {
     static std::atomic<unsigned long long> done{0};
     allow_smem(k_rows_p2<N, L, MODE, FWD>, Tile64<N, L>::smem, done);
-    k_rows_p2<N, L, MODE, FWD><<<(A.count + L - 1) / L, Tile64<N, L>::nt, Tile64<N, L>::smem, st>>>(A);
+    launch_pass(k_rows_p2<N, L, MODE, FWD>, (A.count + L - 1) / L + (A.pairs > 0), Tile64<N, L>::nt,
+                Tile64<N, L>::smem, st, A);
 }
 
 template <int N, int L, int MODE, bool FWD>
@@ -174,7 +189,8 @@ void cols_p2(const Fft64Args &A, cudaStream_t st)
 {
     static std::atomic<unsigned long long> done{0};
     allow_smem(k_cols_p2<N, L, MODE, FWD>, Tile64<N, L>::smem, done);
-    k_cols_p2<N, L, MODE, FWD><<<(A.count + L - 1) / L, Tile64<N, L>::nt, Tile64<N, L>::smem, st>>>(A);
+    launch_pass(k_cols_p2<N, L, MODE, FWD>, (A.count + L - 1) / L + (A.pairs > 0), Tile64<N, L>::nt,
+                Tile64<N, L>::smem, st, A);
 }
 
 // every compiled mode of one length and tile width

@@ -1533,6 +1533,19 @@ void Fused32::check_device_flag()
     }
 }
 
+// The error and the wait flag through pinned memory: one wait for the stream.
+double Fused32::get_error()
+{
+    Impl &I = *impl;
+    volatile double *cell = I.S.err_cell.p;
+    cell[1] = 0;
+    NADIA_CUDA(cudaMemcpyAsync(I.S.err_cell.p, I.S.d_err.p, sizeof(double), cudaMemcpyDeviceToHost, I.S.st));
+    NADIA_CUDA(cudaMemcpyAsync(I.S.err_cell.p + 1, I.flag.p, sizeof(int), cudaMemcpyDeviceToHost, I.S.st));
+    NADIA_CUDA(cudaStreamSynchronize(I.S.st));
+    if (*(volatile int *)(I.S.err_cell.p + 1)) check_device_flag(); // clears it and throws
+    return cell[0];
+}
+
 void Fused32::get_support(double *h) { impl->get_panel(impl->sup.p, 1, h); }
 
 void Fused32::single_op(int, double *)

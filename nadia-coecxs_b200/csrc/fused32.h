@@ -51,6 +51,7 @@ public:
     void autocorrelation(double *out);
     // raise NADIA_ERR_CUDA if a device-side wait of this reconstruction gave up
     void check_device_flag();
+    double get_error();
 
     struct Impl;
     Impl *impl;

@@ -11,6 +11,8 @@
 #include "common.h"
 #include "fft64.h"
 
+#include <vector>
+
 namespace nadia {
 namespace plain {
 
@@ -78,20 +80,24 @@ void poly_scale(double2 *c, const double *isqrt_calc, const double *isqrt,
 // get_2d(MAG), Complex_2D.c++:159-165.
 void magnitude(const double2 *c, double *out, size_t n, cudaStream_t s);
 
-// BaseCDI::convolve, BaseCDI.c++:432-474.  gauss: (cut+1)^2 table (device).
-void convolve(const double *in, double *out, int nx, int ny, const double *gauss, int cut,
+// BaseCDI::convolve with a cut-off of 5 (set_support's soften), BaseCDI.c++:
+// 432-474; g: the (cut+1)^2 weights.
+void convolve(const double *in, double *out, int nx, int ny, const std::vector<double> &g,
               cudaStream_t s);
 
-// Real_2D::get_max, Double_2D.h:252-265 -> *out (device).
-void max_reduce(const double *a, size_t n, double *partials, double *out, cudaStream_t s);
+// the maximum of a non-negative array as its bits, and whether a NaN was seen
+struct Shrink {
+    unsigned long long max;
+    int nan;
+};
 
-// BaseCDI::apply_threshold, BaseCDI.c++:477-492, with its `j < nx` inner
-// bound; *dmax is the maximum taken before thresholding.
-void threshold(double *a, int nx, int ny, double t, const double *dmax, cudaStream_t s);
-
-// out[k] = in[k] / *dmax (BaseCDI::set_support, BaseCDI.c++:95-102).
-void divide_by_max(const double *in, double *out, size_t n, const double *dmax,
-                   cudaStream_t s);
+// BaseCDI::apply_shrinkwrap, BaseCDI.c++:416-429: |x| convolved with a cut-off
+// of 4 (weights g), thresholded at t of its maximum with apply_threshold's
+// `j < nx` bound (BaseCDI.c++:477-492), divided by the maximum of that
+// (set_support, BaseCDI.c++:95-102).  w: four words, zero before the first call;
+// turn: the number of earlier calls with them.
+void shrinkwrap(const double2 *x, double *blurred, double *support, int nx, int ny,
+                const std::vector<double> &g, double t, Shrink *w, int turn, cudaStream_t s);
 
 // FresnelCDI::set_transmission_function, FresnelCDI.c++:253-283 (with its
 // `j < nx` inner bound).

@@ -36,7 +36,7 @@ size_t footprint_bytes(int kind, int nx, int ny, int prec, int n_best, int pad_n
     if (prec == NADIA_FP64) {
         const size_t m = (size_t)std::max(std::max(nx, ny), std::max(pad_nx, pad_ny));
         if (m > plain::kRedBlocks) b += 16 * (m - plain::kRedBlocks); // one error pair per block
-        b += 16;                                          // history counter, ticket
+        b += 8;                                           // history counter
         b += n * (16 + 8 + 8 + 8 + 8); // x, support, sqrt(I), blur result, scratch
         // the combine's projection terms at most; FresnelCDI_WF's second field
         b += (kind != NADIA_FRESNEL_WF ? 4 : 1) * 16 * n;
@@ -45,7 +45,7 @@ size_t footprint_bytes(int kind, int nx, int ny, int prec, int n_best, int pad_n
         // 1021 at most adds as much again)
         b += 16 * (size_t)(2 * (nx + ny) + 4);
         if ((nx | ny) & 1) b += 16 * n; // odd grids: the quadrant swap's gather target
-        b += 8 * 64;                   // blur kernel table
+        b += 64;                       // a shrinkwrap's maxima
         b += (size_t)n_best * 16 * n;
         if (kind == NADIA_FRESNEL) b += 16 * n + 16 * n + 16 * (size_t)(nx / 2) * (ny / 2);
         if (kind == NADIA_FRESNEL_WF) b += 16 * (size_t)(nx / 2) * (ny / 2);

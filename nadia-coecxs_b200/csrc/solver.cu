@@ -72,13 +72,25 @@ private:
     char state_[128];
 };
 
-// Real_2D::get_max, Double_2D.h:252-265
+// Real_2D::get_max, Double_2D.h:252-265: every part starts from the first
+// element, as the whole does
 double host_max(const double *a, size_t n)
 {
     if (n == 0) return 0;
     double m = a[0];
-    for (size_t k = 0; k < n; ++k)
-        if (a[k] > m) m = a[k];
+    std::mutex mu;
+    in_parts(n, [&](size_t from, size_t to) {
+        double p[4] = {a[0], a[0], a[0], a[0]};
+        size_t k = from;
+        for (; k + 4 <= to; k += 4)
+            for (int c = 0; c < 4; ++c)
+                if (a[k + c] > p[c]) p[c] = a[k + c];
+        for (; k < to; ++k)
+            if (a[k] > p[0]) p[0] = a[k];
+        std::lock_guard<std::mutex> lk(mu);
+        for (int c = 0; c < 4; ++c)
+            if (p[c] > m) m = p[c];
+    });
     return m;
 }
 } // namespace
@@ -118,7 +130,6 @@ Solver::Solver(int kind_, int nx_, int ny_, int prec_, int n_best_)
     best_err.assign(n_best, 1.0);   // BaseCDI.c++:48
     best_slot.resize(n_best);
     for (int i = 0; i < n_best; ++i) best_slot[i] = i;
-    dmax.alloc(2);
     if (prec == NADIA_FP64) {
         x.alloc(n);
         support.alloc(n);
@@ -145,14 +156,14 @@ Solver::Solver(int kind_, int nx_, int ny_, int prec_, int n_best_)
     NADIA_CUDA(cudaStreamSynchronize(st));
 }
 
-// FP64: the history's counter, the error sums' ticket and their partials
+// FP64: the history's counter and the error sums' pairs
 void Solver::plain_counters()
 {
     plain_partials((size_t)std::max(nx, ny));
     d_iter.alloc(1);
-    ticket.alloc(1);
     h2d(d_iter.p, &iters, sizeof(iters), st);
-    NADIA_CUDA(cudaMemsetAsync(ticket.p, 0, sizeof(unsigned), st));
+    shrink.alloc(4);
+    NADIA_CUDA(cudaMemsetAsync(shrink.p, 0, shrink.bytes(), st));
 }
 
 // room for one pair of error sums per block
@@ -195,22 +206,6 @@ std::vector<double> Solver::gauss_table(double gauss_width, int cut) const
     return g;
 }
 
-void Solver::plain_convolve(double *arr, double gauss_width, int cut)
-{
-    AllocScope scope(st);
-    // the table stays on the device while the width and cut-off repeat, so
-    // a periodic shrinkwrap neither allocates nor waits for the stream
-    if (!(gauss && gauss_width == gauss_width_ && cut == gauss_cut_)) {
-        std::vector<double> g = gauss_table(gauss_width, cut);
-        gauss.alloc(g.size());
-        h2d(gauss.p, g.data(), g.size() * sizeof(double), st);
-        gauss_width_ = gauss_width;
-        gauss_cut_ = cut;
-    }
-    plain::convolve(arr, tmp.p, nx, ny, gauss.p, cut, st);
-    NADIA_CUDA(cudaMemcpyAsync(arr, tmp.p, n * sizeof(double), cudaMemcpyDeviceToDevice, st));
-}
-
 void Solver::upload_support()
 {
     AllocScope scope(st);
@@ -226,12 +221,15 @@ void Solver::set_support(const double *obj, bool soften)
     AllocScope scope(st);
     ++weights_version;
     double max = host_max(obj, n);
-    for (size_t k = 0; k < n; ++k) h_support[k] = obj[k] / max;
+    in_parts(n, [&](size_t from, size_t to) {
+        for (size_t k = from; k < to; ++k) h_support[k] = obj[k] / max;
+    });
     h_support_valid = true;
     upload_support();
     if (soften) {
         if (prec == NADIA_FP64) {
-            plain_convolve(support.p, 3, 5);
+            plain::convolve(support.p, tmp.p, nx, ny, gauss_table(3, 5), st);
+            std::swap(support, tmp);
         } else {
             f32->soften_support();
         }
@@ -243,7 +241,9 @@ void Solver::set_support(const double *obj, bool soften)
 void Solver::set_intensity(const double *I)
 {
     AllocScope scope(st);
-    for (size_t k = 0; k < n; ++k) h_isqrt[k] = sqrt(I[k]);
+    in_parts(n, [&](size_t from, size_t to) {
+        for (size_t k = from; k < to; ++k) h_isqrt[k] = sqrt(I[k]);
+    });
     if (prec == NADIA_FP64)
         h2d(isqrt.p, h_isqrt.data(), n * sizeof(double), st);
     else
@@ -568,7 +568,10 @@ void Solver::fresnel_wf_set_support(double z_diameter, double size)
         }
     upload_support();
     if (prec == NADIA_FP64)
-        plain_convolve(support.p, 3, 5);
+    {
+        plain::convolve(support.p, tmp.p, nx, ny, gauss_table(3, 5), st);
+        std::swap(support, tmp);
+    }
     else
         f32->soften_support();
     h_support_valid = false;
@@ -830,6 +833,7 @@ void Solver::convert_to_fp64()
         d2h(f.data(), best32[i].p, n * sizeof(float2), st);
         best[i].assign(f.begin(), f.end());
     }
+    d2h(err_cell.p, d_err.p, sizeof(double), st);
     forget_batches_with(uid); // batch plans hold FP32 handles only
     NADIA_CUDA(cudaStreamSynchronize(st));
     const bool had_tc = tc.active;
@@ -846,8 +850,6 @@ void Solver::convert_to_fp64()
     tmp.alloc(n);
     plain_counters();
     fft.init(nx, ny);
-    gauss_width_ = -1;
-    gauss_cut_ = -1;
     h2d(x.p, xh.data(), n * sizeof(double2), st);
     h_support = sup;
     h_support_valid = true;
@@ -975,14 +977,14 @@ void Solver::plain_scale(double2 *c)
     if (kind == NADIA_FRESNEL) {
         // FresnelCDI::scale_intensity, FresnelCDI.c++:217-236
         plain::add_scaled(c, illum.p, 1.0, n, st);
-        plain::scale_intensity(c, isqrt.p, bs_ptr(), n, partials.p, d_err.p, st);
+        plain::scale_intensity(c, isqrt.p, bs_ptr(), n, partials.p, err_cell.p, st);
         plain::add_scaled(c, illum.p, -1.0, n, st);
     } else if (kind == NADIA_POLY) {
         // PolyCDI::scale_intensity, PolyCDI.c++:255-292 (padded field)
         plain::poly_expand(c, d_spec.p, nlambda, lambdac, nx, ny, px, py, isc.p, st);
-        plain::poly_scale(c, isc.p, isqrt.p, bs_ptr(), nx, ny, px, py, partials.p, d_err.p, st);
+        plain::poly_scale(c, isc.p, isqrt.p, bs_ptr(), nx, ny, px, py, partials.p, err_cell.p, st);
     } else {
-        plain::scale_intensity(c, isqrt.p, bs_ptr(), n, partials.p, d_err.p, st);
+        plain::scale_intensity(c, isqrt.p, bs_ptr(), n, partials.p, err_cell.p, st);
     }
 }
 
@@ -1014,8 +1016,12 @@ void Solver::plain_project(double2 *c)
         A.count = nx;
         fft.rows(plain::R_PLAIN, true, A, st);
         A.count = ny;
-        fft.cols(fr ? plain::C_FRESNEL : plain::C_MOD, true, A, st);
-        fft.exec(c, false, st);
+        A.pairs = fft.cols(fr ? plain::C_FRESNEL : plain::C_MOD, true, A, st);
+        A.count = nx;
+        fft.rows(plain::R_PLAIN, false, A, st);
+        A.pairs = 0;
+        A.count = ny;
+        fft.cols(plain::C_PLAIN, false, A, st);
         if (fr) plain::invert(c, nx, ny, true, st);
     } else {
         plain_propagate_to(c, false);
@@ -1045,8 +1051,7 @@ double2 *Solver::second()
 void Solver::error_args(plain::Fft64Args &A, bool record)
 {
     A.partials = partials.p;
-    A.ticket = ticket.p;
-    A.err = d_err.p;
+    A.err = err_cell.p;
     A.ring = record ? d_ring.p : nullptr;
     A.ring_len = kRing;
     A.iter = d_iter.p;
@@ -1107,7 +1112,7 @@ void Solver::fused64_iterate()
         A.calc = isc.p;
         A.lo = A.hi = 0;
         A.count = mx;
-        fft_pad.rows(R_POLY, false, A, st);
+        A.pairs = fft_pad.rows(R_POLY, false, A, st);
         A.first = py;
         A.count = ny;
         fft_pad.cols(C_COMB, false, A, st);
@@ -1127,7 +1132,7 @@ void Solver::fused64_iterate()
             A.src = a;
             A.dst = b;
             A.count = ny;
-            fft.cols(m, fwd, A, st);
+            return fft.cols(m, fwd, A, st);
         };
         rows(R_PLAIN, false, x.p, t);
         cols(C_PLAIN, false, t, t);
@@ -1138,7 +1143,8 @@ void Solver::fused64_iterate()
         cols(C_PLAIN, true, x.p, x.p);
         rows(R_WF_TO, true, x.p, t);
         A.s = 1;
-        cols(C_MOD, true, t, x.p);
+        A.pairs = cols(C_MOD, true, t, x.p);
+        finish_error(A, st);
         return;
     }
     const bool fr = kind == NADIA_FRESNEL;
@@ -1151,9 +1157,10 @@ void Solver::fused64_iterate()
     A.src = P;
     A.count = ny;
     A.swapped = 1; // PlanarCDI's detector is centred; FresnelCDI's estimate is
-    fft.cols(fr ? C_FRESNEL : C_MOD, true, A, st);
+    A.pairs = fft.cols(fr ? C_FRESNEL : C_MOD, true, A, st);
     A.count = nx;
     fft.rows(R_PLAIN, false, A, st);
+    A.pairs = 0;
     A.count = ny;
     A.swapped = fr;
     fft.cols(C_COMB, false, A, st);
@@ -1221,7 +1228,7 @@ void Solver::plain_iterate_once()
 
 void Solver::record_error()
 {
-    plain::record_error(d_err.p, d_ring.p, kRing, d_iter.p, st);
+    plain::record_error(err_cell.p, d_ring.p, kRing, d_iter.p, st);
 }
 
 // BaseCDI::update_n_best, BaseCDI.c++:390-413
@@ -1278,10 +1285,9 @@ void Solver::iterate(int count)
 double Solver::get_error()
 {
     AllocScope scope(st);
-    double e = 0;
-    d2h(&e, d_err.p, sizeof(double), st);
-    if (f32) f32->check_device_flag();
-    return e;
+    if (f32) return f32->get_error();
+    NADIA_CUDA(cudaStreamSynchronize(st));
+    return *(volatile double *)err_cell.p;
 }
 
 void Solver::get_error_history(double *out, int count)
@@ -1305,12 +1311,8 @@ void Solver::apply_shrinkwrap(double gauss_width, double thresh)
         h_support_valid = false;
         return;
     }
-    plain::magnitude(x.p, recon.p, n, st);
-    plain_convolve(recon.p, gauss_width, 4);
-    plain::max_reduce(recon.p, n, partials.p, dmax.p, st);
-    plain::threshold(recon.p, nx, ny, thresh, dmax.p, st);
-    plain::max_reduce(recon.p, n, partials.p, dmax.p + 1, st);
-    plain::divide_by_max(recon.p, support.p, n, dmax.p + 1, st);
+    plain::shrinkwrap(x.p, recon.p, support.p, nx, ny, gauss_table(gauss_width, 4), thresh,
+                      shrink.p, shrinks++, st);
     h_support_valid = false;
     NADIA_CUDA(cudaGetLastError());
 }

@@ -46,11 +46,11 @@ struct Solver {
     // error history: one slot per iteration on the device
     static constexpr int kRing = 65536;
     long long iters = 0;
-    DevBuf<double> d_err;     // [0] current error
+    DevBuf<double> d_err;     // FP32: the current error
+    PinnedCell err_cell;      // FP64: the current error, written by the device
     DevBuf<double> d_ring;    // kRing errors
     DevBuf<double> partials;  // reduction scratch
     DevBuf<long long> d_iter; // FP64: iterations recorded in d_ring
-    DevBuf<unsigned> ticket;  // FP64: blocks of a pass that have left their error sums
 
     // n-best (BaseCDI.c++:43-50, 390-413): slot buffers, rank order, errors
     std::vector<DevBuf<double2>> best64;
@@ -64,9 +64,9 @@ struct Solver {
     double2 *odd_scratch();
     DevBuf<double> support, isqrt, beam_stop;
     plain::Fft2d fft;
-    DevBuf<double> recon, tmp, gauss, dmax;
-    double gauss_width_ = -1; // the blur table now in `gauss`
-    int gauss_cut_ = -1;
+    DevBuf<double> recon, tmp;
+    DevBuf<plain::Shrink> shrink; // the maxima of a shrinkwrap, for two turns
+    int shrinks = 0;
 
     // FresnelCDI
     std::vector<double> h_illum; // detector white field x norm (interleaved)
@@ -161,7 +161,6 @@ struct Solver {
     void plain_propagate_to(double2 *c, bool padded_grid);
     void plain_propagate_from(double2 *c, bool padded_grid);
     void plain_scale(double2 *c);
-    void plain_convolve(double *arr, double gauss_width, int cut);
     void plain_apply_support(double2 *c);
     void apply_transmission_constraint(double2 *t);
 

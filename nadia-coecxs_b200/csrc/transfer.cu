@@ -63,6 +63,48 @@ void PinnedSlots::give(void *p)
     cudaFreeHost(p);
 }
 
+namespace {
+// cells are cut from one slot; it is given back with the slots
+std::vector<double *> &free_cells()
+{
+    static std::vector<double *> *v = new std::vector<double *>;
+    return *v;
+}
+std::vector<void *> &cell_slots()
+{
+    static std::vector<void *> *v = new std::vector<void *>;
+    return *v;
+}
+constexpr size_t kCellBytes = 64;
+size_t g_cells = 0;
+} // namespace
+
+PinnedCell::PinnedCell()
+{
+    std::lock_guard<std::mutex> lk(slot_mu());
+    if (free_cells().empty()) {
+        void *s = nullptr;
+        NADIA_CUDA(cudaHostAlloc(&s, 64 << 10, cudaHostAllocPortable | cudaHostAllocMapped));
+        cell_slots().push_back(s);
+        for (size_t at = 0; at < (64 << 10); at += kCellBytes)
+            free_cells().push_back((double *)((char *)s + at));
+    }
+    p = free_cells().back();
+    free_cells().pop_back();
+    ++g_cells;
+    *p = 0;
+}
+
+PinnedCell::~PinnedCell()
+{
+    std::lock_guard<std::mutex> lk(slot_mu());
+    free_cells().push_back(p);
+    if (--g_cells > 0) return;
+    free_cells().clear();
+    for (void *s : cell_slots()) cudaFreeHost(s);
+    cell_slots().clear();
+}
+
 int borrow_threads(int wanted)
 {
     static const int all = std::max(0, (int)std::thread::hardware_concurrency() / 2);

@@ -44,6 +44,15 @@ private:
 int borrow_threads(int wanted);
 void return_threads(int n);
 
+// A few bytes of pinned memory that the device writes and the host reads.
+struct PinnedCell {
+    double *p; // 0 when made
+    PinnedCell();
+    ~PinnedCell();
+    PinnedCell(const PinnedCell &) = delete;
+    PinnedCell &operator=(const PinnedCell &) = delete;
+};
+
 struct CopySlot {
     void *p = nullptr;
     cudaEvent_t ev = nullptr;
@@ -115,6 +124,30 @@ void in_pieces(int device, size_t rows, size_t row_bytes, Body body)
     for (int i = 0; i < started; ++i) pool[i].join();
     return_threads(extra);
     if (error) std::rethrow_exception(error);
+}
+
+// Calls f(from, to) for parts of 0 .. n-1, several at a time where n is large
+// enough to be worth a thread's start.
+template <class F>
+void in_parts(size_t n, F f)
+{
+    constexpr size_t kPart = 64 << 10;
+    const size_t parts = (n + kPart - 1) / kPart;
+    const int extra = parts > 1 ? borrow_threads((int)std::min<size_t>(7, parts - 1)) : 0;
+    std::atomic<size_t> next{0};
+    auto work = [&] {
+        for (size_t p; (p = next++) < parts;) f(p * kPart, std::min(n, (p + 1) * kPart));
+    };
+    std::thread pool[8];
+    int started = 0;
+    try {
+        for (; started < extra; ++started) pool[started] = std::thread(work);
+    } catch (const std::system_error &) {
+        // fewer threads then
+    }
+    work();
+    for (int i = 0; i < started; ++i) pool[i].join();
+    return_threads(extra);
 }
 
 // Copies that are complete when they return, ordered after the work queued on st.
