@@ -119,13 +119,11 @@ void Fft64Axis::init(int n)
         *p.first = (int)t.size();
         for (int k = 0; k < p.second; ++k) t.push_back(W[(size_t)k * (n / p.second)]);
     }
-    if (plan.np > 0) {
-        int r = plan.pass[0].r1 * plan.pass[0].r2;
-        while (r % 2 == 0) { ++plan.swz; r /= 2; }
-    }
+    const int r0 = plan.np > 0 ? plan.pass[0].r1 * plan.pass[0].r2 : 0;
+    plan.swz = r0 == 8 ? 3 : r0 == 4 ? 2 : 31;
     plan.prime_sm = 1;
     p2 = n >= 64 && n <= 4096 && (n & (n - 1)) == 0;
-    if (smem_any(1) > kSmemMax) plan.prime_sm = 0;
+    if (smem_any(1) > kSmemMax) plan.prime_sm = 0; // the longest lines
     NADIA_REQUIRE(smem_any(1) <= kSmemMax, NADIA_ERR_INVALID, "grid too large for the FP64 transform");
     if (t.empty()) t.push_back(make_double2(1.0, 0.0));
     tw.alloc(t.size());
@@ -150,12 +148,14 @@ int Fft64Axis::tile_p2(int count, bool cols) const
     default: L = cols ? 2 : 1;
     }
     const int least = plan.n <= 128 ? 4 : cols ? 2 : 1;
-    while (L > least && (count + L - 1) / L < 296) L /= 2;
+    // wide column tiles use whole lines, so they give way only to leave no SM idle
+    while (L > least && (count + L - 1) / L < (cols ? 148 : 296)) L /= 2;
     return L;
 }
 
 // Signals and threads to a block of the any-length kernels: the pair with the
-// least estimated time for `count` signals.  A block's time is a latency per
+// least estimated time (in cycles; weights fitted to measurements of all pairs at
+// five sizes on B200, where the pair taken is within 4% of the best one) for `count` signals.  A block's time is a latency per
 // pass and round (a barrier and a trip through shared memory) plus the rounds'
 // work; an SM runs as many blocks as its registers and shared memory hold.
 void Fft64Axis::shape_any(int count, bool cols, int *Lout, int *threads) const
@@ -167,7 +167,7 @@ void Fft64Axis::shape_any(int count, bool cols, int *Lout, int *threads) const
         if (cols && L == 1 && smem_any(2) <= kSmemMax) continue; // half-used sectors
         for (int nt = 64; nt <= kAnyMaxThreads; nt += 32) {
             const int tiles = (count + L - 1) / L;
-            int held = std::min({65536 / (kAnyRegisters * nt), (int)(kSmemMax / (smem + 1024)), 32});
+            int held = std::min({65536 / (kAnyRegisters * nt), (int)((size_t)kAnyCarveKB * 1024 / (smem + 1024)), 32});
             held = std::max(1, std::min(held, (tiles + 147) / 148));
             const int waves = (tiles + 148 * held - 1) / (148 * held);
             double t = 2000 + 2.0 * ((L * plan.n + nt - 1) / nt) * 40; // load and store
@@ -177,9 +177,8 @@ void Fft64Axis::shape_any(int count, bool cols, int *Lout, int *threads) const
                 const bool prime = plan.pass[i].r1 > 8;
                 const int items = prime ? (R + 3) / 4 * L * m : L * m;
                 const int rounds = (items + nt - 1) / nt;
-                const double each = prime ? R * 70.0 : R * 25.0; // cycles of one item
-                t += 400 + rounds * (200 + each);
-                work += rounds * (nt / 32) * (prime ? R * 64.0 : R * 30.0);
+                t += 400 + rounds * (200 + R * (prime ? 130.0 : 25.0));
+                work += prime ? (items + 31) / 32 * R * 64.0 : rounds * (nt / 32) * R * 30.0;
             }
             // four schedulers share the work of the blocks an SM holds
             const double time = waves * std::max(t, held * work / 4);

@@ -174,6 +174,11 @@ __device__ __forceinline__ double2 row_load(const Fft64Args &A, int i, int j, do
 {
     if constexpr (MODE == R_PLAIN) {
         return A.src[(size_t)i * A.ny + j];
+    } else if constexpr (MODE == R_ODD) {
+        const size_t k = (size_t)i * A.ny + j;
+        double2 v = A.src[__ldg(&A.from[k])];
+        for (int c = __ldg(&A.cnt[k]); c > 0; --c) v = make_double2(v.x * A.s, v.y * A.s);
+        return v;
     } else if constexpr (MODE == R_PAD) {
         // i: row of the estimate; the transform's row is i + px
         const int c = j - A.py;

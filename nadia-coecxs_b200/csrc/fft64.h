@@ -11,8 +11,12 @@
 // (32 + 40 + 32 + 56), where one kernel per loop moved about 370.
 //
 // Measured on B200, one HIO iteration, one kernel per loop against this form:
-// 256^2 52 -> 27 us, 1024^2 138 -> 62, 2048^2 468 -> 237, 4096^2 2547 -> 945,
-// 1000x1200 355 -> 154, 515x387 (primes 103 and 43) 2095 -> 232.
+// 128^2 52 -> 16 us, 256^2 52 -> 17, 1024^2 138 -> 45, 2048^2 468 -> 222,
+// 4096^2 2547 -> 916, 1000x1200 355 -> 96, 645x475 (odd) 380 -> 84, 515x387
+// (primes 103 and 43) 2095 -> 123.  What bounds them now: up to 256^2 the four
+// dependent launches; to 1024^2 the latency of one wave of blocks; at 2048^2 the
+// load and store pipe (32-byte pieces of lines in the column passes) and the
+// square root and division of the modulus beside 670 MB of traffic (103 us).
 #pragma once
 
 #include "common.h"
@@ -26,6 +30,7 @@ enum RowMode {
     R_SWAP,    // s * src[p(i, j)]: Complex_2D::invert before FresnelCDI's transform
     R_WF_FROM, // factor(+1) of s * src[p(i, j)] (FresnelCDI_WF::propagate_from_detector)
     R_WF_TO,   // s * factor(-1)(src[p(i, j)])   (FresnelCDI_WF::propagate_to_detector)
+    R_ODD,     // odd grids: the swap loop's replay, s^cnt[k] * src[from[k]]
     R_PAD,     // PolyCDI: row i of the estimate, zero outside columns py..py+ny-1
     R_POLY     // PolyCDI: scale_intensity on s * src, times s; error partials
 };
@@ -58,10 +63,14 @@ struct Fft64Pass {
 
 // the any-length kernels' launch bounds
 constexpr int kAnyMaxThreads = 256, kAnyRegisters = 80;
+// KB of shared memory that their blocks take of an SM's 228 (of which the rest
+// is L1): the twiddles live in L1, and with all 228 taken 1000x1200 took 110 us
+// an iteration and 1080^2 104, with 196 97 and 93, with 132 105 and 109
+constexpr int kAnyCarveKB = 196;
 
 constexpr int kMaxSuper = 14;
 struct Fft64Plan {
-    int n, np, swz; // swz: the first pass's power of two (bank swizzle), 0 for odd
+    int n, np, swz; // swz: 3 or 2 where the first pass is of radix 8 or 4, else 31
     int prime_sm;   // the prime radices' table fits in shared memory
     Fft64Pass pass[kMaxSuper];
 };
@@ -70,7 +79,7 @@ struct Fft64Plan {
 // permutes positions within groups of eight
 __host__ __device__ inline int any_values(int n, int L, int swz)
 {
-    return (swz ? (n + 7) & ~7 : n) * L;
+    return (swz < 31 ? (n + 7) & ~7 : n) * L;
 }
 
 struct Fft64Args {
@@ -83,6 +92,8 @@ struct Fft64Args {
     double s = 1;
     const double *isqrt = nullptr, *bs = nullptr, *sup = nullptr;
     const double2 *coef = nullptr, *ill = nullptr;
+    const int *from = nullptr;  // R_ODD
+    const unsigned char *cnt = nullptr;
     int swapped = 0;            // C_MOD: sqrt(I) at p(q); C_COMB: the value belongs to p(q)
     double2 *x = nullptr;       // C_COMB
     double w[5] = {0, 0, 0, 0, 0}, id = 0;
@@ -159,14 +170,16 @@ void launch_pass(void (*kernel)(P...), int blocks, int threads, size_t smem, cud
 
 // the largest dynamic shared memory a kernel may have, raised once per device
 template <class K>
-void allow_smem(K kernel, size_t bytes, std::atomic<unsigned long long> &done)
+void allow_smem(K kernel, size_t bytes, std::atomic<unsigned long long> &done, int carveout = 0)
 {
-    if (bytes <= 48 * 1024) return;
+    if (bytes <= 48 * 1024 && !carveout) return;
     int dev = 0;
     NADIA_CUDA(cudaGetDevice(&dev));
     const unsigned long long bit = 1ull << (dev & 63);
     if (done.load(std::memory_order_acquire) & bit) return;
     NADIA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    if (carveout)
+        NADIA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, carveout));
     done.fetch_or(bit, std::memory_order_release);
 }
 

@@ -528,14 +528,6 @@ __global__ void k_invert_gather(const double2 *__restrict__ in, double2 *__restr
     }
 }
 
-namespace {
-// the replayed loop of an odd grid: read-only tables, one per device and
-// size, kept for the life of the process (like the twiddle tables)
-struct OddInvert {
-    int *src = nullptr;
-    unsigned char *cnt = nullptr;
-};
-
 const OddInvert &odd_invert(int nx, int ny)
 {
     static std::mutex mu;
@@ -569,7 +561,41 @@ const OddInvert &odd_invert(int nx, int ny)
     }
     return t;
 }
-} // namespace
+
+// Odd grids: the swap and scale_intensity (BaseCDI.c++:163-189) of the detector
+// side, from the transform `in` to the centred field `out`, with the error sums.
+__global__ void k_odd_modulus(const double2 *__restrict__ in, double2 *__restrict__ out,
+                              const int *__restrict__ src, const unsigned char *__restrict__ cnt,
+                              size_t n, double s, const double *__restrict__ isqrt,
+                              const double *__restrict__ bs, double *partials)
+{
+    double diff = 0, mag = 0;
+    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n;
+         k += (size_t)gridDim.x * blockDim.x) {
+        double2 v = in[src[k]];
+        for (int c = cnt[k]; c > 0; --c) v = make_double2(v.x * s, v.y * s);
+        if (bs == nullptr || bs[k] > 0) {
+            const double cis = isqrt[k], cm = mag_of(v);
+            v = set_mag(v, cis);
+            mag += cis * cis;
+            diff += (cm - cis) * (cm - cis);
+        }
+        out[k] = v;
+    }
+    block_sum2(diff, mag);
+    if (threadIdx.x == 0) {
+        partials[2 * blockIdx.x] = diff;
+        partials[2 * blockIdx.x + 1] = mag;
+    }
+}
+
+int odd_modulus(const double2 *in, double2 *out, const OddInvert &t, size_t n, const Fft64Args &A,
+                cudaStream_t s)
+{
+    const int blocks = std::min(grid_of(n), kRedBlocks);
+    k_odd_modulus<<<blocks, kThreads, 0, s>>>(in, out, t.src, t.cnt, n, A.s, A.isqrt, A.bs, A.partials);
+    return blocks;
+}
 
 void invert(double2 *a, int nx, int ny, bool sc, cudaStream_t s, double2 *scratch)
 {

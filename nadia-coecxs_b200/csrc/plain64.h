@@ -25,6 +25,19 @@ constexpr int kRedBlocks = 592;
 // gather into it), unused otherwise
 void invert(double2 *a, int nx, int ny, bool scale, cudaStream_t s, double2 *scratch = nullptr);
 
+// The swap loop replayed for an odd grid: out[k] = in[src[k]] times the scale
+// cnt[k] times.  Read-only tables, one per device and size, kept for the life
+// of the process (like the twiddle tables).
+struct OddInvert {
+    int *src = nullptr;
+    unsigned char *cnt = nullptr;
+};
+const OddInvert &odd_invert(int nx, int ny);
+// the swap and scale_intensity on an odd grid (A: s, isqrt, bs, partials);
+// returns the number of pairs of error sums
+int odd_modulus(const double2 *in, double2 *out, const OddInvert &t, size_t n, const Fft64Args &A,
+                cudaStream_t s);
+
 // BaseCDI::scale_intensity, BaseCDI.c++:163-189.  beam_stop may be null.
 // Writes diff/mag to *err (device).
 void scale_intensity(double2 *c, const double *isqrt, const double *beam_stop, size_t n,
