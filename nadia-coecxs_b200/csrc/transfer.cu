@@ -1,7 +1,10 @@
-// transfer.cu -- pinned slots, the copying threads' budget and plain copies.
+// transfer.cu -- pinned slots, the copying threads and plain copies.
 #include "transfer.h"
 
+#include <condition_variable>
 #include <cstring>
+#include <deque>
+#include <system_error>
 #include <vector>
 
 namespace nadia {
@@ -19,7 +22,7 @@ std::vector<void *> &free_slots()
     return *v;
 }
 size_t g_users = 0;
-std::atomic<int> g_threads{0};
+void end_helpers();
 } // namespace
 
 PinnedSlots::User::User()
@@ -30,10 +33,13 @@ PinnedSlots::User::User()
 
 PinnedSlots::User::~User()
 {
-    std::lock_guard<std::mutex> lk(slot_mu());
-    if (--g_users > 0) return;
-    for (void *p : free_slots()) cudaFreeHost(p);
-    free_slots().clear();
+    {
+        std::lock_guard<std::mutex> lk(slot_mu());
+        if (--g_users > 0) return;
+        for (void *p : free_slots()) cudaFreeHost(p);
+        free_slots().clear();
+    }
+    end_helpers();
 }
 
 void *PinnedSlots::take()
@@ -105,17 +111,91 @@ PinnedCell::~PinnedCell()
     cell_slots().clear();
 }
 
-int borrow_threads(int wanted)
+namespace {
+// one with_helpers call: helpers it still wants, and those at work in it
+struct Task {
+    const std::function<void()> *f;
+    int want, running;
+};
+// leaked on purpose, like the slots
+struct Helpers {
+    std::mutex mu;
+    std::condition_variable wake, done;
+    std::vector<std::thread> threads;
+    std::deque<Task *> tasks;
+    bool stop = false;
+};
+Helpers &helpers()
 {
-    static const int all = std::max(0, (int)std::thread::hardware_concurrency() / 2);
-    int have = g_threads.load();
+    static Helpers *h = new Helpers;
+    return *h;
+}
+void help()
+{
+    Helpers &h = helpers();
+    std::unique_lock<std::mutex> lk(h.mu);
     for (;;) {
-        const int n = std::max(0, std::min(wanted, all - have));
-        if (g_threads.compare_exchange_weak(have, have + n)) return n;
+        h.wake.wait(lk, [&] { return h.stop || !h.tasks.empty(); });
+        if (h.stop) return;
+        Task *t = h.tasks.front();
+        if (--t->want == 0) h.tasks.pop_front();
+        ++t->running;
+        lk.unlock();
+        (*t->f)();
+        lk.lock();
+        if (--t->running == 0) h.done.notify_all();
     }
 }
+void end_helpers()
+{
+    Helpers &h = helpers();
+    std::vector<std::thread> old;
+    {
+        std::lock_guard<std::mutex> lk(h.mu);
+        if (!h.tasks.empty()) return; // a call without a reconstruction is at work
+        h.stop = true;
+        old.swap(h.threads);
+    }
+    h.wake.notify_all();
+    for (std::thread &t : old) t.join();
+    std::lock_guard<std::mutex> lk(h.mu);
+    h.stop = false;
+}
+} // namespace
 
-void return_threads(int n) { g_threads -= n; }
+void with_helpers(int extra, const std::function<void()> &f)
+{
+    static const int most = (int)std::thread::hardware_concurrency() / 2;
+    extra = std::min(extra, most);
+    if (extra <= 0) {
+        f();
+        return;
+    }
+    Helpers &h = helpers();
+    Task t{&f, extra, 0};
+    {
+        std::lock_guard<std::mutex> lk(h.mu);
+        if (h.stop) t.want = 0;
+        try {
+            while (!h.stop && (int)h.threads.size() < most) h.threads.emplace_back(help);
+        } catch (const std::system_error &) {
+            // fewer helpers then
+        }
+        if (t.want > 0) h.tasks.push_back(&t);
+    }
+    if (extra == 1)
+        h.wake.notify_one();
+    else
+        h.wake.notify_all();
+    f();
+    std::unique_lock<std::mutex> lk(h.mu);
+    for (auto it = h.tasks.begin(); it != h.tasks.end(); ++it)
+        if (*it == &t) {
+            h.tasks.erase(it);
+            break;
+        }
+    h.done.wait(lk, [&] { return t.running == 0; });
+}
 
 namespace {
 constexpr size_t kRow = 64 << 10;      // plain copies are cut in "rows" of this size

@@ -11,8 +11,8 @@
 
 #include <algorithm>
 #include <exception>
+#include <functional>
 #include <mutex>
-#include <system_error>
 #include <thread>
 
 #include "common.h"
@@ -39,10 +39,12 @@ private:
     static constexpr size_t kKeep = 16;
 };
 
-// threads that copies of this process may use now beside their callers:
-// half the cores between all concurrent copies
-int borrow_threads(int wanted);
-void return_threads(int n);
+// Runs f on the calling thread and on up to `extra` helper threads at once;
+// returns when all have returned.  f divides its work among its callers itself
+// and does not throw.  The helpers are the process's (half its cores at most,
+// shared by all concurrent calls; starting threads for each call instead cost
+// about 0.1 ms), sleep between calls and end with the last reconstruction.
+void with_helpers(int extra, const std::function<void()> &f);
 
 // A few bytes of pinned memory that the device writes and the host reads.
 struct PinnedCell {
@@ -93,18 +95,17 @@ void in_pieces(int device, size_t rows, size_t row_bytes, Body body)
     // two pieces a thread at least, and pieces worth a thread's start
     const size_t worth = std::max<size_t>(1, (1u << 20) / row_bytes);
     const int most = (int)std::min<size_t>(8, rows / worth + 1);
-    const int extra = borrow_threads(most - 1);
-    const size_t per = std::max<size_t>(1, std::min(fit, (rows + 2 * (extra + 1) - 1) / (2 * (extra + 1))));
+    const size_t per = std::max<size_t>(1, std::min(fit, (rows + 2 * most - 1) / (2 * most)));
     std::atomic<size_t> next{0};
     std::exception_ptr error;
     std::mutex mu;
     auto work = [&](bool own) {
         try {
             if (!own) NADIA_CUDA(cudaSetDevice(device));
+            size_t r = next.fetch_add(per);
+            if (r >= rows) return; // the others were quicker
             CopySlot slot;
-            for (;;) {
-                const size_t r = next.fetch_add(per);
-                if (r >= rows) break;
+            for (; r < rows; r = next.fetch_add(per)) {
                 body(slot, r, std::min(per, rows - r));
             }
         } catch (...) {
@@ -113,16 +114,8 @@ void in_pieces(int device, size_t rows, size_t row_bytes, Body body)
             if (!error) error = std::current_exception();
         }
     };
-    std::thread pool[8];
-    int started = 0;
-    try {
-        for (; started < extra; ++started) pool[started] = std::thread(work, false);
-    } catch (const std::system_error &) {
-        // fewer threads then
-    }
-    work(true);
-    for (int i = 0; i < started; ++i) pool[i].join();
-    return_threads(extra);
+    const std::thread::id caller = std::this_thread::get_id();
+    with_helpers(most - 1, [&] { work(std::this_thread::get_id() == caller); });
     if (error) std::rethrow_exception(error);
 }
 
@@ -133,21 +126,10 @@ void in_parts(size_t n, F f)
 {
     constexpr size_t kPart = 64 << 10;
     const size_t parts = (n + kPart - 1) / kPart;
-    const int extra = parts > 1 ? borrow_threads((int)std::min<size_t>(7, parts - 1)) : 0;
     std::atomic<size_t> next{0};
-    auto work = [&] {
+    with_helpers((int)std::min<size_t>(7, parts - (parts > 0)), [&] {
         for (size_t p; (p = next++) < parts;) f(p * kPart, std::min(n, (p + 1) * kPart));
-    };
-    std::thread pool[8];
-    int started = 0;
-    try {
-        for (; started < extra; ++started) pool[started] = std::thread(work);
-    } catch (const std::system_error &) {
-        // fewer threads then
-    }
-    work();
-    for (int i = 0; i < started; ++i) pool[i].join();
-    return_threads(extra);
+    });
 }
 
 // Copies that are complete when they return, ordered after the work queued on st.
