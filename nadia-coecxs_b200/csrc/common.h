@@ -138,6 +138,25 @@ inline void upload_now(void *dst, const void *src, size_t bytes)
     NADIA_CUDA(cudaStreamSynchronize(0));
 }
 
+// Launches a pass so that it may start while the work before it on st drains
+// (the kernel waits for that before it touches global memory).
+template <class... P, class... V>
+void launch_pass(void (*kernel)(P...), dim3 blocks, int threads, size_t smem, cudaStream_t st,
+                 const V &...args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = blocks;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    NADIA_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+}
+
 constexpr int kMaxPasses = 40;
 constexpr int kMaxRadix = 64;    // generic radices up to this keep their inputs in registers
 constexpr int kMaxPrime = 1021;  // the largest prime factor a transform length may have

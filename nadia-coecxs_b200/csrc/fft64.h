@@ -149,25 +149,6 @@ struct Fft2d {
 // the error metric from `pairs` pairs of sums, where no pass follows
 void finish_error(const Fft64Args &A, cudaStream_t s);
 
-// launches a pass so that it may start while the work before it on st drains
-// (the kernel waits for it, see after_previous)
-template <class... P, class... V>
-void launch_pass(void (*kernel)(P...), int blocks, int threads, size_t smem, cudaStream_t st,
-                 const V &...args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)blocks);
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    NADIA_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
-}
-
 // the largest dynamic shared memory a kernel may have, raised once per device
 template <class K>
 void allow_smem(K kernel, size_t bytes, std::atomic<unsigned long long> &done, int carveout = 0)

@@ -1032,13 +1032,20 @@ void Fused32::Impl::flush_intensity()
     mI_dirty = false;
     std::vector<float> &m = mstage; // kept between calls, like the staging array
     m.resize(n);
+    // the sum by fixed parts, added in order (the same on every machine)
+    std::vector<double> sums((n + kPart - 1) / kPart, 0.0);
+    in_parts(n, [&](size_t from, size_t to) {
+        double norm2 = 0;
+        for (size_t d = from; d < to; ++d) {
+            const bool measured = !S.has_beam_stop || h_bs[d] > 0;
+            const float v = (float)S.h_isqrt[d];
+            if (measured) norm2 += (double)v * (double)v;
+            m[d] = measured ? v : -1.f;
+        }
+        sums[from / kPart] = norm2;
+    });
     double norm2 = 0;
-    for (size_t d = 0; d < n; ++d) {
-        const bool measured = !S.has_beam_stop || h_bs[d] > 0;
-        const float v = (float)S.h_isqrt[d];
-        if (measured) norm2 += (double)v * (double)v;
-        m[d] = measured ? v : -1.f;
-    }
+    for (double v : sums) norm2 += v;
     // PlanarCDI's detector is centred (Complex_2D::invert): fold it into
     // transform order; Fresnel folds the swap into its phase factors, and
     // PolyCDI gathers in centred coordinates
@@ -1112,11 +1119,13 @@ void Fused32::set_fresnel_geometry(double factor)
     const int qy = I.ny / 2;
     double x_mid = (I.nx - 1) / 2.0, y_mid = (I.ny - 1) / 2.0;
     std::vector<double2> hc((size_t)(I.nx / 2) * qy);
-    for (int i = 0; i < I.nx / 2; i++)
-        for (int j = 0; j < qy; j++) {
+    in_parts(hc.size(), [&](size_t from, size_t to) {
+        for (size_t k = from; k < to; ++k) {
+            const int i = (int)(k / qy), j = (int)(k % qy);
             double phi = factor * ((x_mid - i) * (x_mid - i) + (y_mid - j) * (y_mid - j));
-            hc[(size_t)i * qy + j] = make_double2(cos(phi), sin(phi));
+            hc[k] = make_double2(cos(phi), sin(phi));
         }
+    });
     DevBuf<double2> coef(hc.size()), c(I.n);
     plain::Fft2d fft;
     fft.init(I.nx, I.ny);
@@ -1360,7 +1369,7 @@ void Fused32::Impl::launch_iteration_wf(cudaStream_t st)
     const Slot *const *sl = slot_ptr.p;
     wfc->wf_col(sl, 1, nx, ny, twx, st);
     wfr->wf_row(kRowFull, sl, 1, nx, ny, twy, st);
-    k_wf_finish<256><<<1, 256, 0, st>>>(sl);
+    launch_pass(k_wf_finish<256>, 1, 256, 0, st, sl);
 }
 
 void Fused32::Impl::launch_iteration(cudaStream_t st)

@@ -156,6 +156,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_col(const Slot *const *slots
                                                const float2 *__restrict__ tw)
 {
     extern __shared__ float2 sm[];
+    after_previous();
     const Slot &S = *slots[blockIdx.y];
     float2 *__restrict__ P = S.P;
     const float *__restrict__ mI = S.mI;
@@ -203,6 +204,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_col(const Slot *const *slots
     if (threadIdx.x == 0) S.partials[blockIdx.x] = tot;
 
     transform<C, false>(v, sm, tw);
+    let_next_start();
     for_each_slot<C, false, false>([&](int e, int s, int pos) {
         P[paddr(pos, c0 * kPanel + s, nx)] = v[e];
     });
@@ -248,6 +250,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_row(const Slot *const *slots
                                                const float2 *__restrict__ tw)
 {
     extern __shared__ float2 sm[];
+    after_previous();
     const Slot &S = *slots[blockIdx.y];
     float2 *__restrict__ P = S.P;
     float2 *__restrict__ x = S.x;
@@ -336,6 +339,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_row(const Slot *const *slots
         });
     }
     transform<C, true>(v, sm, tw);
+    let_next_start();
     for_each_slot<C, true, false>([&](int e, int s, int pos) {
         P[paddr(i0 + s, pos, nx)] = v[e];
     });
@@ -388,16 +392,16 @@ void launch_row_tc(int half, const Slot *const *slots, int nslots, int nx, int n
 {
     const dim3 grid(nx / C::L, nslots);
     if (half == 1)
-        k_row_tc<C, 1><<<grid, C::NT, smem_bytes<C>(), st>>>(slots, nx, ny, tw);
+        launch_pass(k_row_tc<C, 1>, grid, C::NT, smem_bytes<C>(), st, slots, nx, ny, tw);
     else
-        k_row_tc<C, 2><<<grid, C::NT, smem_bytes<C>(), st>>>(slots, nx, ny, tw);
+        launch_pass(k_row_tc<C, 2>, grid, C::NT, smem_bytes<C>(), st, slots, nx, ny, tw);
 }
 
 template <class C>
 void launch_wf_col(const Slot *const *slots, int nslots, int nx, int ny, const float2 *tw,
                    cudaStream_t st)
 {
-    k_wf_col<C><<<dim3(ny / C::L, nslots), C::NT, smem_bytes<C>(), st>>>(slots, nx, ny, tw);
+    launch_pass(k_wf_col<C>, dim3(ny / C::L, nslots), C::NT, smem_bytes<C>(), st, slots, nx, ny, tw);
 }
 
 template <class C>
@@ -406,9 +410,9 @@ void launch_wf_row(int mode, const Slot *const *slots, int nslots, int nx, int n
 {
     const dim3 grid(nx / C::L, nslots);
     if (mode == kRowFull)
-        k_wf_row<C, kRowFull><<<grid, C::NT, smem_bytes<C>(), st>>>(slots, nx, ny, tw);
+        launch_pass(k_wf_row<C, kRowFull>, grid, C::NT, smem_bytes<C>(), st, slots, nx, ny, tw);
     else
-        k_wf_row<C, kRowPrime><<<grid, C::NT, smem_bytes<C>(), st>>>(slots, nx, ny, tw);
+        launch_pass(k_wf_row<C, kRowPrime>, grid, C::NT, smem_bytes<C>(), st, slots, nx, ny, tw);
 }
 
 template <class C>
@@ -417,9 +421,9 @@ void launch_col(bool fresnel, const Slot *const *slots, int nslots, int nx, int 
 {
     dim3 grid(ny / C::L, nslots);
     if (fresnel)
-        k_col<C, true><<<grid, C::NT, smem_bytes<C>(), st>>>(slots, nx, ny, tw);
+        launch_pass(k_col<C, true>, grid, C::NT, smem_bytes<C>(), st, slots, nx, ny, tw);
     else
-        k_col<C, false><<<grid, C::NT, smem_bytes<C>(), st>>>(slots, nx, ny, tw);
+        launch_pass(k_col<C, false>, grid, C::NT, smem_bytes<C>(), st, slots, nx, ny, tw);
 }
 
 template <class C>
@@ -429,16 +433,16 @@ void launch_row(int mode, const Slot *const *slots, int nslots, int nx, int ny, 
     dim3 grid(nx / C::L, nslots);
     switch (mode) {
     case kRowFull:
-        k_row<C, kRowFull><<<grid, C::NT, smem_bytes<C>(), st>>>(slots, nx, ny, tw);
+        launch_pass(k_row<C, kRowFull>, grid, C::NT, smem_bytes<C>(), st, slots, nx, ny, tw);
         break;
     case kRowPrime:
-        k_row<C, kRowPrime><<<grid, C::NT, smem_bytes<C>(), st>>>(slots, nx, ny, tw);
+        launch_pass(k_row<C, kRowPrime>, grid, C::NT, smem_bytes<C>(), st, slots, nx, ny, tw);
         break;
     case kRowPfs:
-        k_row<C, kRowPfs><<<grid, C::NT, smem_bytes<C>(), st>>>(slots, nx, ny, tw);
+        launch_pass(k_row<C, kRowPfs>, grid, C::NT, smem_bytes<C>(), st, slots, nx, ny, tw);
         break;
     default:
-        k_row<C, kRowPrimePfs><<<grid, C::NT, smem_bytes<C>(), st>>>(slots, nx, ny, tw);
+        launch_pass(k_row<C, kRowPrimePfs>, grid, C::NT, smem_bytes<C>(), st, slots, nx, ny, tw);
     }
 }
 
@@ -510,9 +514,9 @@ void launch_col_persistent(bool fresnel, const Slot *const *slots, int nslots, i
     const int cap = sm_count() * PersistCol<C, STAGES, MMODE>::per_sm;
     const int grid = ntiles < cap ? ntiles : cap;
     if (fresnel)
-        kp_col<C, true, STAGES, MMODE><<<grid, C::NT, bytes, st>>>(slots, nslots, nx, ny, tw);
+        launch_pass(kp_col<C, true, STAGES, MMODE>, grid, C::NT, bytes, st, slots, nslots, nx, ny, tw);
     else
-        kp_col<C, false, STAGES, MMODE><<<grid, C::NT, bytes, st>>>(slots, nslots, nx, ny, tw);
+        launch_pass(kp_col<C, false, STAGES, MMODE>, grid, C::NT, bytes, st, slots, nslots, nx, ny, tw);
 }
 
 template <class C>
@@ -526,7 +530,7 @@ void launch_row_persistent(int mode, const Slot *const *slots, int nslots, int n
     const int ntiles = (nx / C::L) * nslots;
     const int cap = sm_count() * PersistRow<C>::per_sm;
     const int grid = ntiles < cap ? ntiles : cap;
-    kp_row<C><<<grid, C::NT, persist_row_smem<C>(), st>>>(slots, nslots, nx, ny, tw);
+    launch_pass(kp_row<C>, grid, C::NT, persist_row_smem<C>(), st, slots, nslots, nx, ny, tw);
 }
 
 // One tile shape (N, NT threads, L signals per block, radices, swizzle, min
@@ -568,11 +572,9 @@ void launch_col_staged(bool fresnel, const Slot *const *slots, int nslots, int n
 {
     dim3 grid(ny / C::L, nslots);
     if (fresnel)
-        k_col<C, true, true><<<grid, C::NT, smem_bytes<C>() + col_stage_bytes<C, true>(), st>>>(
-            slots, nx, ny, tw);
+        launch_pass(k_col<C, true, true>, grid, C::NT, smem_bytes<C>() + col_stage_bytes<C, true>(), st, slots, nx, ny, tw);
     else
-        k_col<C, false, true><<<grid, C::NT, smem_bytes<C>() + col_stage_bytes<C, false>(), st>>>(
-            slots, nx, ny, tw);
+        launch_pass(k_col<C, false, true>, grid, C::NT, smem_bytes<C>() + col_stage_bytes<C, false>(), st, slots, nx, ny, tw);
 }
 
 template <int N, int NT, int L, int MINB, class SW, bool PING, int... Rs>
@@ -732,7 +734,7 @@ void launch_row_grouped(int mode, const Slot *const *slots, int nslots, int nx, 
     const int ntiles = (nx / C::L) * nslots;
     const int ctas = (ntiles + C::GROUPS - 1) / C::GROUPS;
     const int grid = ctas < sm_count() ? ctas : sm_count();
-    kg_row<C><<<grid, C::NT * C::GROUPS, grouped_row_smem<C>(), st>>>(slots, nslots, nx, ny, tw);
+    launch_pass(kg_row<C>, grid, C::NT * C::GROUPS, grouped_row_smem<C>(), st, slots, nslots, nx, ny, tw);
 }
 
 template <class C>
@@ -752,9 +754,9 @@ void launch_col_grouped(bool fresnel, const Slot *const *slots, int nslots, int 
     const int ctas = (ntiles + C::GROUPS - 1) / C::GROUPS;
     const int grid = ctas < sm_count() ? ctas : sm_count();
     if (fresnel)
-        kg_col<C, true><<<grid, C::NT * C::GROUPS, grouped_col_smem<C>(), st>>>(slots, nslots, nx, ny, tw);
+        launch_pass(kg_col<C, true>, grid, C::NT * C::GROUPS, grouped_col_smem<C>(), st, slots, nslots, nx, ny, tw);
     else
-        kg_col<C, false><<<grid, C::NT * C::GROUPS, grouped_col_smem<C>(), st>>>(slots, nslots, nx, ny, tw);
+        launch_pass(kg_col<C, false>, grid, C::NT * C::GROUPS, grouped_col_smem<C>(), st, slots, nslots, nx, ny, tw);
 }
 
 // The column pass in G independent groups of NT threads a CTA, each on half

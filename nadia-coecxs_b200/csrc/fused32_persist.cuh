@@ -95,6 +95,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB)
         tma::fence_barrier_init();
     }
     __syncthreads();
+    after_previous();
 
     // the first tile's reconstruction sets the wait limit (and the test hook
     // that leaves the first tile's copy unissued, see Slot::skip_first_load)
@@ -208,6 +209,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB)
         }
 
         transform_h<C, false>(v, Pb, Xb, tw, [] {});
+        if (tn >= ntiles) let_next_start();
         for_each_slot<C, false, false>([&](int e, int s, int pos) { Pb[raw_col<C>(s, pos)] = v[e]; });
         tma::fence_async_shared();
         __syncthreads();
@@ -264,6 +266,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB)
         tma::mbar_init(&bar[2], 1);
         tma::fence_barrier_init();
     }
+    after_previous();
     // slots whose error this CTA finishes (the column pass ran before)
     for (int sl = blockIdx.x; sl < nslots; sl += gridDim.x) finish_error<C::NT>(*slots[sl]);
     __syncthreads();
@@ -341,6 +344,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB)
             v[e] = xn;
         });
         transform<C, true>(v, Pb, tw);
+        if (tn >= ntiles) let_next_start();
         for_each_slot<C, true, false>([&](int e, int s, int pos) { Pb[raw_row<C>(s, pos)] = v[e]; });
         tma::fence_async_shared();
         if (__syncthreads_or(!okx)) {
@@ -421,6 +425,7 @@ __global__ void __launch_bounds__(C::NT * C::GROUPS, 1)
         tma::mbar_init(&bar[2], 1);
         tma::fence_barrier_init();
     }
+    after_previous();
     // slots whose error this CTA finishes (the column pass ran before)
     for (int sl = blockIdx.x; sl < nslots; sl += gridDim.x) finish_error<C::NT * G>(*slots[sl]);
     __syncthreads();
@@ -500,6 +505,7 @@ __global__ void __launch_bounds__(C::NT * C::GROUPS, 1)
             v[e] = xn;
         });
         transform<C, true>(v, Pb, tw);
+        if (tn >= ntiles) let_next_start();
         for_each_slot<C, true, false>([&](int e, int s, int pos) { Pb[raw_row<C>(s, pos)] = v[e]; });
         tma::fence_async_shared();
         if (group_or<C>(!okx)) {
@@ -576,6 +582,7 @@ __global__ void __launch_bounds__(C::NT * C::GROUPS, 1)
         tma::fence_barrier_init();
     }
     __syncthreads();
+    after_previous();
 
     int t = blockIdx.x * G + g;
     const int stride = gridDim.x * G;
@@ -664,6 +671,7 @@ __global__ void __launch_bounds__(C::NT * C::GROUPS, 1)
             }
         }
         transform<C, false>(v, Pb, tw);
+        if (tn >= ntiles) let_next_start();
         for_each_slot<C, false, false>([&](int e, int s, int pos) { Pb[pos * 2 + s] = v[e]; });
         tma::fence_async_shared();
         C::sync();

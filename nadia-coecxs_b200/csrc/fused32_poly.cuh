@@ -44,6 +44,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_poly_col_fwd(const Slot *con
                                                                    const float2 *__restrict__ tw)
 {
     extern __shared__ float2 sm[];
+    after_previous();
     const Slot &S = *slots[blockIdx.y];
     float2 *__restrict__ P = S.P;
     const int mx = S.mx, my = S.my, r0 = S.px, r1 = S.mx - S.px; // the estimate's rows
@@ -54,6 +55,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_poly_col_fwd(const Slot *con
                                        : make_float2(0.f, 0.f);
     });
     transform<C, true>(v, sm, tw);
+    let_next_start();
     const float s02 = S.s0 * S.s0;
     float *__restrict__ q = S.q;
     for_each_slot<C, true, false>([&](int e, int s, int kx) {
@@ -79,6 +81,7 @@ constexpr int kNoSample = -(1 << 30); // offset of a sample outside the padded g
 // elsewhere; partials[block] = sum of (sqrt(I) - sqrt(I_calc))^2.
 __global__ void __launch_bounds__(kExpandThreads) k_poly_expand(const Slot *const *slots)
 {
+    after_previous();
     const Slot &S = *slots[blockIdx.y];
     const int mx = S.mx, px = S.px, py = S.py;
     const int nx = mx - 2 * px, ny = S.my - 2 * py;
@@ -185,6 +188,7 @@ __global__ void __launch_bounds__(kExpandThreads) k_poly_expand(const Slot *cons
         ratio[a] = r;
     }
     }
+    let_next_start();
     const double tot = block_sum<kExpandThreads>(diff);
     if (threadIdx.x == 0) S.partials[blockIdx.x] = tot;
 }
@@ -194,6 +198,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_poly_col_inv(const Slot *con
                                                                    const float2 *__restrict__ tw)
 {
     extern __shared__ float2 sm[];
+    after_previous();
     const Slot &S = *slots[blockIdx.y];
     float2 *__restrict__ P = S.P;
     const int mx = S.mx, my = S.my, px = S.px, py = S.py;
@@ -210,6 +215,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_poly_col_inv(const Slot *con
         v[e] = cscale(P[paddr(kx, ky, mx)], s02 * r);
     });
     transform<C, false>(v, sm, tw);
+    let_next_start();
     for_each_slot<C, false, false>([&](int e, int s, int pos) {
         if (pos >= px && pos < px + nx) P[paddr(pos, c0 * kPanel + s, mx)] = v[e];
     });
@@ -233,6 +239,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_poly_row(const Slot *const *
                                                                const float2 *__restrict__ tw)
 {
     extern __shared__ float2 sm[];
+    after_previous();
     const Slot &S = *slots[blockIdx.y];
     float2 *__restrict__ P = S.P;
     float2 *__restrict__ x = S.x;
@@ -314,6 +321,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_poly_row(const Slot *const *
         });
     }
     transform<C, true>(v, sm, tw);
+    let_next_start();
     for_each_slot<C, true, false>([&](int e, int s, int pos) {
         P[paddr(px + i0 + s, pos, mx)] = v[e];
     });
@@ -335,15 +343,15 @@ template <class C>
 void launch_poly_col_fwd(const Slot *const *slots, int nslots, int tiles, cudaStream_t st,
                          const float2 *tw)
 {
-    k_poly_col_fwd<C><<<dim3(tiles, nslots), C::NT, smem_bytes<C>(), st>>>(slots, tw);
+    launch_pass(k_poly_col_fwd<C>, dim3(tiles, nslots), C::NT, smem_bytes<C>(), st, slots, tw);
 }
 
 template <class C>
 void launch_poly_col_inv(const Slot *const *slots, int nslots, int tiles, cudaStream_t st,
                          const float2 *tw)
 {
-    k_poly_expand<<<dim3(kExpandBlocks, nslots), kExpandThreads, 0, st>>>(slots);
-    k_poly_col_inv<C><<<dim3(tiles, nslots), C::NT, smem_bytes<C>(), st>>>(slots, tw);
+    launch_pass(k_poly_expand, dim3(kExpandBlocks, nslots), kExpandThreads, 0, st, slots);
+    launch_pass(k_poly_col_inv<C>, dim3(tiles, nslots), C::NT, smem_bytes<C>(), st, slots, tw);
 }
 
 template <class C, bool PREF>
@@ -351,10 +359,11 @@ void launch_poly_row(int mode, const Slot *const *slots, int nslots, int tiles, 
                      const float2 *tw)
 {
     if (mode == kRowFull)
-        k_poly_row<C, kRowFull, PREF>
-            <<<dim3(tiles, nslots), C::NT, poly_row_smem<C, PREF>(), st>>>(slots, tw);
+        launch_pass(k_poly_row<C, kRowFull, PREF>, dim3(tiles, nslots), C::NT, poly_row_smem<C, PREF>(),
+                    st, slots, tw);
     else
-        k_poly_row<C, kRowPrime, PREF><<<dim3(tiles, nslots), C::NT, smem_bytes<C>(), st>>>(slots, tw);
+        launch_pass(k_poly_row<C, kRowPrime, PREF>, dim3(tiles, nslots), C::NT, smem_bytes<C>(), st,
+                    slots, tw);
 }
 
 template <int N, int NT, int L, int MINB, class SW, int... Rs>

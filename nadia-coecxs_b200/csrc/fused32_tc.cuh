@@ -95,6 +95,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_row_tc(const Slot *const *sl
                                                   const float2 *__restrict__ tw)
 {
     extern __shared__ float2 sm[];
+    after_previous();
     const Slot &S = *slots[blockIdx.y];
     float2 *__restrict__ P = S.P;
     float2 *__restrict__ Y = S.Y;

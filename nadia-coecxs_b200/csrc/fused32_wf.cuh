@@ -65,6 +65,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_wf_col(const Slot *const *sl
                                                   const float2 *__restrict__ tw)
 {
     extern __shared__ float2 sm[];
+    after_previous();
     const Slot &S = *slots[blockIdx.y];
     float2 *__restrict__ P = S.P;
     const float2 *__restrict__ bx = S.tx;
@@ -76,17 +77,17 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_wf_col(const Slot *const *sl
         const float2 a = P[paddr(i, y0 + s, nx)];
         v[e] = make_float2(a.x, -a.y);
     });
-    transform<C, true>(v, sm, tw);
+    transform<Scalar<C>, true>(v, sm, tw);
     for_each_slot<C, true, false>([&](int e, int, int k) { v[e] = conj_mul(v[e], __ldg(&bx[k])); });
-    transform<C, false>(v, sm, tw);
+    transform<Scalar<C>, false>(v, sm, tw);
     // c4 -> c5: BaseCDI::support_constraint (BaseCDI.c++:136-154)
     for_each_slot<C, false, false>([&](int e, int s, int i) {
-        v[e] = cscale(v[e], support_factor(__ldg(&sup[paddr(i, y0 + s, nx)])));
+        v[e] = cscale<false>(v[e], support_factor(__ldg(&sup[paddr(i, y0 + s, nx)])));
     });
-    transform<C, true>(v, sm, tw);
+    transform<Scalar<C>, true>(v, sm, tw);
     // times conj(b_x), then the forward transform as conj(I(conj v))
     for_each_slot<C, true, false>([&](int e, int, int k) { v[e] = conj_mul(v[e], __ldg(&bx[k])); });
-    transform<C, false>(v, sm, tw);
+    transform<Scalar<C>, false>(v, sm, tw);
     for_each_slot<C, false, false>([&](int e, int s, int i) {
         P[paddr(i, y0 + s, nx)] = make_float2(v[e].x, -v[e].y);
     });
@@ -101,6 +102,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_wf_row(const Slot *const *sl
                                                   const float2 *__restrict__ tw)
 {
     extern __shared__ float2 sm[];
+    after_previous();
     const Slot &S = *slots[blockIdx.y];
     float2 *__restrict__ P = S.P;
     float2 *__restrict__ x = S.x;
@@ -109,9 +111,9 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_wf_row(const Slot *const *sl
     float2 v[C::E];
     if (MODE == kRowFull) {
         for_each_slot<C, true, true>([&](int e, int s, int j) { v[e] = P[paddr(i0 + s, j, nx)]; });
-        transform<C, true>(v, sm, tw);
+        transform<Scalar<C>, true>(v, sm, tw);
         for_each_slot<C, true, false>([&](int e, int, int k) { v[e] = conj_mul(v[e], __ldg(&by[k])); });
-        transform<C, false>(v, sm, tw);
+        transform<Scalar<C>, false>(v, sm, tw);
         const float *__restrict__ mI = S.mI;
         double diff = 0.0;
         for_each_slot<C, false, false>([&](int e, int s, int j) {
@@ -130,9 +132,10 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_wf_row(const Slot *const *sl
             v[e] = make_float2(sg * c.x, -sg * c.y);
         });
     }
-    transform<C, true>(v, sm, tw);
+    transform<Scalar<C>, true>(v, sm, tw);
     for_each_slot<C, true, false>([&](int e, int, int k) { v[e] = conj_mul(v[e], __ldg(&by[k])); });
-    transform<C, false>(v, sm, tw);
+    transform<Scalar<C>, false>(v, sm, tw);
+    let_next_start();
     for_each_slot<C, false, false>([&](int e, int s, int j) { P[paddr(i0 + s, j, nx)] = v[e]; });
 }
 
@@ -141,6 +144,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_wf_row(const Slot *const *sl
 template <int NT>
 __global__ void __launch_bounds__(NT) k_wf_finish(const Slot *const *slots)
 {
+    after_previous();
     finish_error_row<NT>(*slots[blockIdx.x]);
 }
 

@@ -121,10 +121,10 @@ void in_pieces(int device, size_t rows, size_t row_bytes, Body body)
 
 // Calls f(from, to) for parts of 0 .. n-1, several at a time where n is large
 // enough to be worth a thread's start.
+constexpr size_t kPart = 64 << 10; // values of a part
 template <class F>
 void in_parts(size_t n, F f)
 {
-    constexpr size_t kPart = 64 << 10;
     const size_t parts = (n + kPart - 1) / kPart;
     std::atomic<size_t> next{0};
     with_helpers((int)std::min<size_t>(7, parts - (parts > 0)), [&] {
