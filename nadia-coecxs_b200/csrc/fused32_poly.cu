@@ -8,25 +8,24 @@
 
 #include "batch.h"
 #include "fused32.h"
-#include "fused32_poly.cuh"
+#include "fused32_poly3.cuh"
 #include "solver.h"
 
 namespace nadia {
 namespace f32 {
 
 // Padded sizes with PolyCDI tiles: 256 and 512 (small cases) and 1080, the
-// 1024 x 1024 detector padded by 28 on each side (1080 = 6*6*6*5, so every
-// radix divides the 30 values a thread holds).  A 1080-point tile needs
-// about 168 registers a thread, so an SM holds 288 such threads: as one CTA
-// of 8 signals, or as two independent CTAs of 4 signals and 144 threads
-// (four and a half warps), whose global loads and barriers overlap each
-// other's arithmetic.  Swizzles from tests/swizzle_search.py.
+// 1024 x 1024 detector padded by 28 on each side.  1080 points run on tiles of
+// one butterfly a thread (fused32_poly3.cuh); the tiles of 30 values a thread
+// (6*6*6*5, 168 registers: 288 threads an SM, as one block or two) remain for
+// comparison (NADIA_POLY_TILE).  Swizzles from tests/swizzle_search.py.
 const std::vector<PolyVariant> &poly_variants(int n)
 {
     static const std::map<int, std::vector<PolyVariant>> reg = [] {
         std::map<int, std::vector<PolyVariant>> r;
         r[256].push_back(make_poly<256, 256, 8, 3, Swizzle<4, 6, 3, 2>, 8, 8, 4>("8.8.4"));
         r[512].push_back(make_poly<512, 256, 8, 2, Swizzle<4, 6, 3, 2>, 16, 8, 4>("16.8.4"));
+        r[1080].push_back(make_poly3<Tile3<1080, 10, 12, 9, 2>>("10.12.9"));
         r[1080].push_back(make_poly<1080, 144, 4, 2, Swizzle<7, 0, 7, 1>, 6, 6, 6, 5>("6.6.6.5"));
         r[1080].push_back(
             make_poly<1080, 144, 4, 2, Swizzle<7, 0, 7, 1>, 6, 6, 6, 5>("6.6.6.5 direct", false));
