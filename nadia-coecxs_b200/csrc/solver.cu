@@ -345,8 +345,10 @@ void Solver::fresnel_init(const double *wf, double wl, double zfd_, double zfs_,
 {
     AllocScope scope(st);
     norm = norm_;
-    h_illum.assign(2 * n, 0.0);
-    for (size_t k = 0; k < 2 * n; ++k) h_illum[k] = wf[k] * norm;
+    h_illum.resize(2 * n);
+    in_parts(2 * n, [&](size_t from, size_t to) {
+        for (size_t k = from; k < to; ++k) h_illum[k] = wf[k] * norm;
+    });
     if (prec == NADIA_FP64) {
         illum.alloc(n);
         illum_sample.alloc(n);
@@ -373,11 +375,14 @@ void Solver::fresnel_set_experimental_parameters(double wl, double zfd_, double 
     double zsd = zfd - zfs;
     double factor = pixel * pixel * M_PI / (wavelength) * ((1 / zfd) - (1 / zsd));
     std::vector<double2> hc((size_t)(nx / 2) * qy);
-    for (int i = 0; i < nx / 2; i++)
-        for (int j = 0; j < qy; j++) {
-            double phi = factor * ((x_mid - i) * (x_mid - i) + (y_mid - j) * (y_mid - j));
-            hc[(size_t)i * qy + j] = make_double2(cos(phi), sin(phi));
-        }
+    if (prec == NADIA_FP64) // the FP32 form makes its own factors per axis
+        in_parts(hc.size(), [&](size_t from, size_t to) {
+            for (size_t k = from; k < to; ++k) {
+                const int i = (int)(k / qy), j = (int)(k % qy);
+                double phi = factor * ((x_mid - i) * (x_mid - i) + (y_mid - j) * (y_mid - j));
+                hc[k] = make_double2(cos(phi), sin(phi));
+            }
+        });
     if (prec == NADIA_FP64) {
         h2d(coef.p, hc.data(), coef.bytes(), st);
         NADIA_CUDA(cudaMemcpyAsync(illum_sample.p, illum.p, n * sizeof(double2),
