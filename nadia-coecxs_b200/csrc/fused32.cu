@@ -918,105 +918,89 @@ void Fused32::Impl::prepare_pfs()
     if (!pfs_choice) pfs_choice = &choose(nx, ny, S.kind == NADIA_FRESNEL, 1, true);
 }
 
-// Rows r0 .. r0+rows-1 of an array in the reference's order (element (x, y) at
-// x*ny + y), in mapped host memory, to or from the panel layout.  A thread
-// moves 16 bytes: STRIDE neighbouring ones are four columns of a panel row.
-// The host side of the transfer crosses the link as full warps' runs of 512
-// bytes, so the order costs no pass of its own on either side.  `fold` moves
-// PlanarCDI's centred detector to transform order.
-template <int STRIDE>
-__global__ void k_panel_put(const float4 *__restrict__ h, float4 *__restrict__ d, int nx, int ny,
-                            int r0, int rows, int fold)
-{
-    const int q = ny / kPanel * STRIDE; // 16-byte units of a row
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < rows * q; e += gridDim.x * blockDim.x) {
-        int x = r0 + e / q;
-        const int f = e % q, half = f % STRIDE;
-        int p = f / STRIDE;
-        if (fold) { // source (dx, dy) belongs at (dx + nx/2, dy + ny/2)
-            x += nx / 2;
-            x = x >= nx ? x - nx : x;
-            p += ny / kPanel / 2;
-            p = p >= ny / kPanel ? p - ny / kPanel : p;
-        }
-        d[((size_t)p * nx + x) * STRIDE + half] = __ldcs(&h[e]);
-    }
-}
-
-template <int STRIDE>
-__global__ void k_panel_get(const float4 *__restrict__ d, float4 *__restrict__ h, int nx, int ny,
-                            int r0, int rows)
-{
-    const int q = ny / kPanel * STRIDE;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < rows * q; e += gridDim.x * blockDim.x) {
-        const int x = r0 + e / q, f = e % q, p = f / STRIDE, half = f % STRIDE;
-        __stcs(&h[e], d[((size_t)p * nx + x) * STRIDE + half]);
-    }
-}
-
 namespace {
-// blocks of a piece's reordering kernel: enough to fill the link, few enough
-// to leave the GPU to other reconstructions' passes
-constexpr int kPanelBlocks = 64, kPanelThreads = 512;
-
-template <class T>
-void put_rows(const T *h, int stride, void *dst, bool fold, int nx, int ny, int device,
+// Rows r0 .. r0+rows-1 of a panel-layout array: one run of rows*kPanel elements
+// per panel, so a piece of whole rows is one 2-D copy of the copy engines and
+// never waits for SMs held by other reconstructions' passes, as a kernel that
+// reorders while it crosses the link does.  The host threads make the order,
+// four elements at a time, from a slot that stays in their caches.  B200, 16
+// estimates of 2048^2 read and set again beside a running batch of 16: 90 ms
+// (269 ms converted by one thread a handle); one estimate alone read in 1.0 ms
+// into a warm buffer, set in 1.1 ms.
+template <int stride, class T>
+void put_rows(const T *h, void *dst, bool fold, int nx, int ny, int device,
               cudaStream_t st)
 {
     const size_t w = (size_t)ny * stride;
+    constexpr int q = kPanel * stride; // values of a panel row
+    const int np = ny / kPanel;
+    const size_t run = (size_t)q * sizeof(float);
     in_pieces(device, nx, w * sizeof(float), [&](CopySlot &slot, size_t r0, size_t rows) {
         float *p = static_cast<float *>(slot.p);
-        const T *src = h + r0 * w;
-        for (size_t k = 0; k < rows * w; ++k) p[k] = (float)src[k];
-        if (stride == 1)
-            k_panel_put<1><<<kPanelBlocks, kPanelThreads, 0, st>>>(
-                (const float4 *)p, (float4 *)dst, nx, ny, (int)r0, (int)rows, fold);
-        else
-            k_panel_put<2><<<kPanelBlocks, kPanelThreads, 0, st>>>(
-                (const float4 *)p, (float4 *)dst, nx, ny, (int)r0, (int)rows, fold);
-        NADIA_CUDA(cudaGetLastError());
+        for (size_t x = 0; x < rows; ++x) {
+            // row x of the piece is row r0 + x of the device array
+            size_t dx = r0 + x;
+            if (fold) dx = dx + nx / 2 >= (size_t)nx ? dx + nx / 2 - nx : dx + nx / 2;
+            const T *src = h + dx * w;
+            for (int k = 0; k < np; ++k) {
+                const int from = fold ? (k + np / 2 >= np ? k + np / 2 - np : k + np / 2) : k;
+                float *d = p + ((size_t)k * rows + x) * q;
+                const T *v = src + (size_t)from * q;
+                for (int c = 0; c < q; ++c) d[c] = (float)v[c];
+            }
+        }
+        NADIA_CUDA(cudaMemcpy2DAsync((char *)dst + r0 * run, (size_t)nx * run, p, rows * run,
+                                     rows * run, np, cudaMemcpyHostToDevice, st));
         slot.wait(st);
     });
 }
 
-template <class T>
-void get_rows(const void *src, int stride, T *h, int nx, int ny, int device, cudaStream_t st)
+template <int stride, class T>
+void get_rows(const void *src, T *h, int nx, int ny, int device, cudaStream_t st)
 {
     const size_t w = (size_t)ny * stride;
+    constexpr int q = kPanel * stride;
+    const int np = ny / kPanel;
+    const size_t run = (size_t)q * sizeof(float);
     in_pieces(device, nx, w * sizeof(float), [&](CopySlot &slot, size_t r0, size_t rows) {
         const float *p = static_cast<const float *>(slot.p);
-        if (stride == 1)
-            k_panel_get<1><<<kPanelBlocks, kPanelThreads, 0, st>>>(
-                (const float4 *)src, (float4 *)slot.p, nx, ny, (int)r0, (int)rows);
-        else
-            k_panel_get<2><<<kPanelBlocks, kPanelThreads, 0, st>>>(
-                (const float4 *)src, (float4 *)slot.p, nx, ny, (int)r0, (int)rows);
-        NADIA_CUDA(cudaGetLastError());
+        NADIA_CUDA(cudaMemcpy2DAsync(slot.p, rows * run, (const char *)src + r0 * run,
+                                     (size_t)nx * run, rows * run, np, cudaMemcpyDeviceToHost, st));
         slot.wait(st);
-        T *dst = h + r0 * w;
-        for (size_t k = 0; k < rows * w; ++k) dst[k] = (T)p[k];
+        for (size_t x = 0; x < rows; ++x) {
+            T *dst = h + (r0 + x) * w;
+            for (int k = 0; k < np; ++k) {
+                const float *v = p + ((size_t)k * rows + x) * q;
+                T *d = dst + (size_t)k * q;
+                for (int c = 0; c < q; ++c) d[c] = (T)v[c];
+            }
+        }
     });
 }
 } // namespace
 
 void Fused32::Impl::put_panel_f(const float *h, int stride, void *dst, bool fold)
 {
-    put_rows(h, stride, dst, fold, nx, ny, S.device, S.st);
+    stride == 1 ? put_rows<1>(h, dst, fold, nx, ny, S.device, S.st)
+                : put_rows<2>(h, dst, fold, nx, ny, S.device, S.st);
 }
 
 void Fused32::Impl::put_panel(const double *h, int stride, void *dst, bool fold)
 {
-    put_rows(h, stride, dst, fold, nx, ny, S.device, S.st);
+    stride == 1 ? put_rows<1>(h, dst, fold, nx, ny, S.device, S.st)
+                : put_rows<2>(h, dst, fold, nx, ny, S.device, S.st);
 }
 
 void Fused32::Impl::get_panel_f(const void *src, int stride, float *h)
 {
-    get_rows(src, stride, h, nx, ny, S.device, S.st);
+    stride == 1 ? get_rows<1>(src, h, nx, ny, S.device, S.st)
+                : get_rows<2>(src, h, nx, ny, S.device, S.st);
 }
 
 void Fused32::Impl::get_panel(const void *src, int stride, double *h)
 {
-    get_rows(src, stride, h, nx, ny, S.device, S.st);
+    stride == 1 ? get_rows<1>(src, h, nx, ny, S.device, S.st)
+                : get_rows<2>(src, h, nx, ny, S.device, S.st);
 }
 
 // set_intensity and set_beam_stop mark sqrt(I) for conversion; it is formed

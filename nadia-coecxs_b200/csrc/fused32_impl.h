@@ -294,8 +294,8 @@ struct Fused32::Impl {
     void use_ncol(int ncol) { h_slot.ncol = ncol; } // column tiles the row pass sums over
     // host arrays in the reference's order <-> device arrays in the panel
     // layout (stride 1: real, 2: complex; fold: PlanarCDI's centred detector
-    // to transform order): through pinned slots (transfer.h), the host threads
-    // converting the values and a kernel the order
+    // to transform order): through pinned slots (transfer.h), converted by the
+    // host threads
     std::vector<float> mstage; // sqrt(I) with the unmeasured pixels marked, kept between calls
     void put_panel(const double *h, int stride, void *dst, bool fold);
     void put_panel_f(const float *h, int stride, void *dst, bool fold);

@@ -16,10 +16,22 @@ std::mutex &slot_mu()
     static std::mutex *m = new std::mutex;
     return *m;
 }
-std::vector<void *> &free_slots()
+struct Arena {
+    void *base = nullptr;
+    std::vector<void *> free;
+    std::condition_variable given;
+    void release() // with slot_mu held; only when every slot is back
+    {
+        if (!base || free.size() < (size_t)kSlots) return;
+        cudaFreeHost(base);
+        base = nullptr;
+        free.clear();
+    }
+};
+Arena &arena()
 {
-    static std::vector<void *> *v = new std::vector<void *>;
-    return *v;
+    static Arena *a = new Arena;
+    return *a;
 }
 size_t g_users = 0;
 void end_helpers();
@@ -36,37 +48,34 @@ PinnedSlots::User::~User()
     {
         std::lock_guard<std::mutex> lk(slot_mu());
         if (--g_users > 0) return;
-        for (void *p : free_slots()) cudaFreeHost(p);
-        free_slots().clear();
+        arena().release();
     }
     end_helpers();
 }
 
 void *PinnedSlots::take()
 {
-    {
-        std::lock_guard<std::mutex> lk(slot_mu());
-        if (!free_slots().empty()) {
-            void *p = free_slots().back();
-            free_slots().pop_back();
-            return p;
-        }
+    std::unique_lock<std::mutex> lk(slot_mu());
+    Arena &A = arena();
+    if (!A.base) {
+        void *p = nullptr;
+        NADIA_CUDA(cudaHostAlloc(&p, kSlots * kSlotBytes, cudaHostAllocPortable));
+        A.base = p;
+        for (int k = 0; k < kSlots; ++k) A.free.push_back((char *)p + k * kSlotBytes);
     }
-    void *p = nullptr;
-    NADIA_CUDA(cudaHostAlloc(&p, kSlotBytes, cudaHostAllocPortable | cudaHostAllocMapped));
+    A.given.wait(lk, [&] { return !A.free.empty(); });
+    void *p = A.free.back();
+    A.free.pop_back();
     return p;
 }
 
 void PinnedSlots::give(void *p)
 {
-    {
-        std::lock_guard<std::mutex> lk(slot_mu());
-        if (g_users > 0 && free_slots().size() < kKeep) {
-            free_slots().push_back(p);
-            return;
-        }
-    }
-    cudaFreeHost(p);
+    std::lock_guard<std::mutex> lk(slot_mu());
+    Arena &A = arena();
+    A.free.push_back(p);
+    A.given.notify_one();
+    if (g_users == 0) A.release();
 }
 
 namespace {

@@ -19,10 +19,14 @@
 
 namespace nadia {
 
-constexpr size_t kSlotBytes = 4u << 20; // one pinned slot
+constexpr size_t kSlotBytes = 2u << 20; // one pinned slot
+constexpr int kSlots = 16;
 
-// Pinned slots of the process: at most kKeep unused ones are kept, and none
-// once the last reconstruction is gone.
+// Pinned slots of the process, made together at the first transfer and given
+// back when the last reconstruction is gone; a thread that finds none free waits
+// for one.  (Making or freeing pinned memory waits for the whole device: with
+// slots made as they ran short, 16 threads reading estimates beside a running
+// batch waited for its end.)
 class PinnedSlots {
 public:
     // held by every reconstruction
@@ -34,9 +38,6 @@ public:
     };
     static void *take();
     static void give(void *p);
-
-private:
-    static constexpr size_t kKeep = 16;
 };
 
 // Runs f on the calling thread and on up to `extra` helper threads at once;
