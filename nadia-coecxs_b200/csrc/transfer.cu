@@ -1,10 +1,8 @@
-// transfer.cu -- pinned slots, the copying threads and plain copies.
+// transfer.cu -- pinned slots and plain copies.
 #include "transfer.h"
 
 #include <condition_variable>
 #include <cstring>
-#include <deque>
-#include <system_error>
 #include <vector>
 
 namespace nadia {
@@ -34,7 +32,6 @@ Arena &arena()
     return *a;
 }
 size_t g_users = 0;
-void end_helpers();
 } // namespace
 
 PinnedSlots::User::User()
@@ -45,12 +42,9 @@ PinnedSlots::User::User()
 
 PinnedSlots::User::~User()
 {
-    {
-        std::lock_guard<std::mutex> lk(slot_mu());
-        if (--g_users > 0) return;
-        arena().release();
-    }
-    end_helpers();
+    std::lock_guard<std::mutex> lk(slot_mu());
+    if (--g_users > 0) return;
+    arena().release();
 }
 
 void *PinnedSlots::take()
@@ -118,92 +112,6 @@ PinnedCell::~PinnedCell()
     free_cells().clear();
     for (void *s : cell_slots()) cudaFreeHost(s);
     cell_slots().clear();
-}
-
-namespace {
-// one with_helpers call: helpers it still wants, and those at work in it
-struct Task {
-    const std::function<void()> *f;
-    int want, running;
-};
-// leaked on purpose, like the slots
-struct Helpers {
-    std::mutex mu;
-    std::condition_variable wake, done;
-    std::vector<std::thread> threads;
-    std::deque<Task *> tasks;
-    bool stop = false;
-};
-Helpers &helpers()
-{
-    static Helpers *h = new Helpers;
-    return *h;
-}
-void help()
-{
-    Helpers &h = helpers();
-    std::unique_lock<std::mutex> lk(h.mu);
-    for (;;) {
-        h.wake.wait(lk, [&] { return h.stop || !h.tasks.empty(); });
-        if (h.stop) return;
-        Task *t = h.tasks.front();
-        if (--t->want == 0) h.tasks.pop_front();
-        ++t->running;
-        lk.unlock();
-        (*t->f)();
-        lk.lock();
-        if (--t->running == 0) h.done.notify_all();
-    }
-}
-void end_helpers()
-{
-    Helpers &h = helpers();
-    std::vector<std::thread> old;
-    {
-        std::lock_guard<std::mutex> lk(h.mu);
-        if (!h.tasks.empty()) return; // a call without a reconstruction is at work
-        h.stop = true;
-        old.swap(h.threads);
-    }
-    h.wake.notify_all();
-    for (std::thread &t : old) t.join();
-    std::lock_guard<std::mutex> lk(h.mu);
-    h.stop = false;
-}
-} // namespace
-
-void with_helpers(int extra, const std::function<void()> &f)
-{
-    static const int most = (int)std::thread::hardware_concurrency() / 2;
-    extra = std::min(extra, most);
-    if (extra <= 0) {
-        f();
-        return;
-    }
-    Helpers &h = helpers();
-    Task t{&f, extra, 0};
-    {
-        std::lock_guard<std::mutex> lk(h.mu);
-        if (h.stop) t.want = 0;
-        try {
-            while (!h.stop && (int)h.threads.size() < most) h.threads.emplace_back(help);
-        } catch (const std::system_error &) {
-            // fewer helpers then
-        }
-        if (t.want > 0) h.tasks.push_back(&t);
-    }
-    if (extra == 1)
-        h.wake.notify_one();
-    else
-        h.wake.notify_all();
-    f();
-    std::unique_lock<std::mutex> lk(h.mu);
-    for (auto it = h.tasks.begin(); it != h.tasks.end(); ++it)
-        if (*it == &t) {
-            h.tasks.erase(it);
-            break;
-        }
-    h.done.wait(lk, [&] { return t.running == 0; });
 }
 
 namespace {

@@ -11,11 +11,11 @@
 
 #include <algorithm>
 #include <exception>
-#include <functional>
 #include <mutex>
 #include <thread>
 
 #include "common.h"
+#include "helpers.h"
 
 namespace nadia {
 
@@ -31,6 +31,7 @@ class PinnedSlots {
 public:
     // held by every reconstruction
     struct User {
+        HelperUse helpers;
         User();
         ~User();
         User(const User &) = delete;
@@ -39,13 +40,6 @@ public:
     static void *take();
     static void give(void *p);
 };
-
-// Runs f on the calling thread and on up to `extra` helper threads at once;
-// returns when all have returned.  f divides its work among its callers itself
-// and does not throw.  The helpers are the process's (half its cores at most,
-// shared by all concurrent calls; starting threads for each call instead cost
-// about 0.1 ms), sleep between calls and end with the last reconstruction.
-void with_helpers(int extra, const std::function<void()> &f);
 
 // A few bytes of pinned memory that the device writes and the host reads.
 struct PinnedCell {
