@@ -126,7 +126,7 @@ void to_device(void *d, const void *h, size_t bytes, int device, cudaStream_t st
         NADIA_CUDA(cudaStreamSynchronize(st));
         return;
     }
-    in_pieces(device, (bytes + kRow - 1) / kRow, kRow, [&](CopySlot &slot, size_t r, size_t rows) {
+    in_pieces(device, st, (bytes + kRow - 1) / kRow, kRow, [&](CopySlot &slot, size_t r, size_t rows) {
         const size_t at = r * kRow, len = std::min(rows * kRow, bytes - at);
         std::memcpy(slot.p, (const char *)h + at, len);
         NADIA_CUDA(cudaMemcpyAsync((char *)d + at, slot.p, len, cudaMemcpyHostToDevice, st));
@@ -141,7 +141,7 @@ void to_host(void *h, const void *d, size_t bytes, int device, cudaStream_t st)
         NADIA_CUDA(cudaStreamSynchronize(st));
         return;
     }
-    in_pieces(device, (bytes + kRow - 1) / kRow, kRow, [&](CopySlot &slot, size_t r, size_t rows) {
+    in_pieces(device, st, (bytes + kRow - 1) / kRow, kRow, [&](CopySlot &slot, size_t r, size_t rows) {
         const size_t at = r * kRow, len = std::min(rows * kRow, bytes - at);
         NADIA_CUDA(cudaMemcpyAsync(slot.p, (const char *)d + at, len, cudaMemcpyDeviceToHost, st));
         slot.wait(st);

@@ -70,7 +70,8 @@ struct CopySlot {
     }
     CopySlot(const CopySlot &) = delete;
     CopySlot &operator=(const CopySlot &) = delete;
-    // waits until what was queued on st by now is done
+    // waits until what was queued on st by now is done: one piece's copy (the
+    // event is polled, as tens of microseconds are too short to sleep)
     void wait(cudaStream_t st)
     {
         NADIA_CUDA(cudaEventRecord(ev, st));
@@ -81,11 +82,18 @@ struct CopySlot {
 // Calls body(slot, first row, rows) for pieces of `rows` rows of `row_bytes`
 // (as they pass through a slot); each piece is done when its call returns.
 // The first error of any thread is thrown once all have stopped.
+//
+// The calling thread waits for the work queued on st before any slot or helper
+// is taken, so that those are held for copies only: a read behind long
+// iterations otherwise held eight of the sixteen slots until they ended, and a
+// few such reads kept every other reconstruction's transfers waiting (and each
+// of their threads polling) although its own stream was idle.
 template <class Body>
-void in_pieces(int device, size_t rows, size_t row_bytes, Body body)
+void in_pieces(int device, cudaStream_t st, size_t rows, size_t row_bytes, Body body)
 {
     NADIA_REQUIRE(row_bytes <= kSlotBytes, NADIA_ERR_INVALID, "row too long to transfer");
     if (rows == 0) return;
+    NADIA_CUDA(cudaStreamSynchronize(st));
     const size_t fit = kSlotBytes / row_bytes;
     // two pieces a thread at least, and pieces worth a thread's start
     const size_t worth = std::max<size_t>(1, (1u << 20) / row_bytes);
