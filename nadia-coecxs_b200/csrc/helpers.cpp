@@ -40,6 +40,7 @@ struct Helpers {
     std::vector<std::thread> threads; // those at work or asleep
     std::vector<std::thread> ended;   // to be joined, which does not wait
     std::deque<Task *> tasks;
+    std::vector<void (*)()> give_back; // by the last helper to end
     size_t uses = 0;
     Clock::time_point unused_since = Clock::now();
     bool closed = false; // the process (or the library) ends; never lowered
@@ -67,19 +68,30 @@ void help()
 {
     Helpers &h = helpers();
     std::unique_lock<std::mutex> lk(h.mu);
+    bool given = false;
     for (;;) {
         if (h.closed) return;
         if (h.tasks.empty()) {
+            const Clock::time_point until = h.unused_since + kHelperLinger;
             if (h.uses > 0) {
+                given = false;
                 h.wake.wait(lk);
                 continue;
             }
-            const Clock::time_point until = h.unused_since + kHelperLinger;
             if (Clock::now() < until) {
+                given = false;
                 h.wake.wait_until(lk, until);
                 continue;
             }
             // unused for long enough
+            if (h.threads.size() == 1 && !given) {
+                const std::vector<void (*)()> fs = h.give_back;
+                lk.unlock();
+                for (void (*f)() : fs) f();
+                lk.lock();
+                given = true;
+                continue; // unless there is a user again
+            }
             for (std::thread &t : h.threads)
                 if (t.get_id() == std::this_thread::get_id()) {
                     h.ended.push_back(std::move(t));
@@ -139,8 +151,21 @@ HelperUse::~HelperUse()
         std::lock_guard<std::mutex> lk(h.mu);
         if (--h.uses > 0) return;
         h.unused_since = Clock::now();
+        try {
+            // there is one to give things back
+            if (!h.closed && h.threads.empty() && !h.give_back.empty()) h.threads.emplace_back(help);
+        } catch (...) {
+            // they stay until the next time
+        }
     }
     h.wake.notify_all(); // from now on they sleep for a limited time
+}
+
+void when_unused(void (*give_back)())
+{
+    Helpers &h = helpers();
+    std::lock_guard<std::mutex> lk(h.mu);
+    h.give_back.push_back(give_back);
 }
 
 void with_helpers(int extra, const std::function<void()> &f)

@@ -22,4 +22,9 @@ public:
 // about 0.1 ms).
 void with_helpers(int extra, const std::function<void()> &f);
 
+// give_back() is called on a helper thread when there has been no reconstruction
+// for kHelperLinger: what the process keeps from one reconstruction to the next
+// ends there.  Call it once for each function.
+void when_unused(void (*give_back)());
+
 } // namespace nadia

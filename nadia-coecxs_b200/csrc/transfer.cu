@@ -3,115 +3,136 @@
 
 #include <condition_variable>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 namespace nadia {
 
 namespace {
-// leaked on purpose: reconstructions destroyed by static destructors still use them
-std::mutex &slot_mu()
-{
-    static std::mutex *m = new std::mutex;
-    return *m;
-}
-struct Arena {
+// Making and freeing pinned memory is refused to a thread (and breaks the
+// capture) while another thread captures a graph in the global mode, unless
+// this thread says that it does not take part.
+struct NoCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    NoCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~NoCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+constexpr size_t kCellBytes = 64, kCellBlock = 64 << 10;
+
+struct Pinned {
+    std::mutex mu;
+    size_t users = 0;
+    int device = 0; // whose context the memory was made in
+    // the slots, made together
     void *base = nullptr;
     std::vector<void *> free;
     std::condition_variable given;
-    void release() // with slot_mu held; only when every slot is back
+    // the cells, cut from blocks
+    std::vector<void *> blocks;
+    std::vector<double *> free_cells;
+    size_t cells = 0;
+
+    void *make(size_t bytes) // with mu held
     {
-        if (!base || free.size() < (size_t)kSlots) return;
-        cudaFreeHost(base);
-        base = nullptr;
-        free.clear();
+        NoCapture guard;
+        void *p = nullptr;
+        NADIA_CUDA(cudaGetDevice(&device));
+        NADIA_CUDA(cudaHostAlloc(&p, bytes, cudaHostAllocPortable | cudaHostAllocMapped));
+        return p;
     }
 };
-Arena &arena()
+void give_back();
+// leaked on purpose: reconstructions destroyed by static destructors still use it
+Pinned &pinned()
 {
-    static Arena *a = new Arena;
-    return *a;
+    static Pinned *p = [] {
+        when_unused(give_back);
+        return new Pinned;
+    }();
+    return *p;
 }
-size_t g_users = 0;
+
+// on a helper thread, some time after the last reconstruction
+void give_back()
+{
+    Pinned &P = pinned();
+    std::lock_guard<std::mutex> lk(P.mu);
+    if (P.users > 0) return;
+    NoCapture guard;
+    if ((P.base || !P.blocks.empty()) && cudaSetDevice(P.device) != cudaSuccess) return;
+    if (P.base && P.free.size() == (size_t)kSlots) {
+        cudaFreeHost(P.base);
+        P.base = nullptr;
+        P.free.clear();
+    }
+    if (P.cells == 0) {
+        for (void *b : P.blocks) cudaFreeHost(b);
+        P.blocks.clear();
+        P.free_cells.clear();
+    }
+}
 } // namespace
 
 PinnedSlots::User::User()
 {
-    std::lock_guard<std::mutex> lk(slot_mu());
-    ++g_users;
+    Pinned &P = pinned();
+    std::lock_guard<std::mutex> lk(P.mu);
+    ++P.users;
 }
 
 PinnedSlots::User::~User()
 {
-    std::lock_guard<std::mutex> lk(slot_mu());
-    if (--g_users > 0) return;
-    arena().release();
+    Pinned &P = pinned();
+    std::lock_guard<std::mutex> lk(P.mu);
+    --P.users;
 }
 
 void *PinnedSlots::take()
 {
-    std::unique_lock<std::mutex> lk(slot_mu());
-    Arena &A = arena();
-    if (!A.base) {
-        void *p = nullptr;
-        NADIA_CUDA(cudaHostAlloc(&p, kSlots * kSlotBytes, cudaHostAllocPortable));
-        A.base = p;
-        for (int k = 0; k < kSlots; ++k) A.free.push_back((char *)p + k * kSlotBytes);
+    Pinned &P = pinned();
+    std::unique_lock<std::mutex> lk(P.mu);
+    if (!P.base) {
+        void *p = P.make(kSlots * kSlotBytes);
+        P.base = p;
+        for (int k = 0; k < kSlots; ++k) P.free.push_back((char *)p + k * kSlotBytes);
     }
-    A.given.wait(lk, [&] { return !A.free.empty(); });
-    void *p = A.free.back();
-    A.free.pop_back();
+    P.given.wait(lk, [&] { return !P.free.empty(); });
+    void *p = P.free.back();
+    P.free.pop_back();
     return p;
 }
 
 void PinnedSlots::give(void *p)
 {
-    std::lock_guard<std::mutex> lk(slot_mu());
-    Arena &A = arena();
-    A.free.push_back(p);
-    A.given.notify_one();
-    if (g_users == 0) A.release();
+    Pinned &P = pinned();
+    std::lock_guard<std::mutex> lk(P.mu);
+    P.free.push_back(p);
+    P.given.notify_one();
 }
-
-namespace {
-// cells are cut from one slot; it is given back with the slots
-std::vector<double *> &free_cells()
-{
-    static std::vector<double *> *v = new std::vector<double *>;
-    return *v;
-}
-std::vector<void *> &cell_slots()
-{
-    static std::vector<void *> *v = new std::vector<void *>;
-    return *v;
-}
-constexpr size_t kCellBytes = 64;
-size_t g_cells = 0;
-} // namespace
 
 PinnedCell::PinnedCell()
 {
-    std::lock_guard<std::mutex> lk(slot_mu());
-    if (free_cells().empty()) {
-        void *s = nullptr;
-        NADIA_CUDA(cudaHostAlloc(&s, 64 << 10, cudaHostAllocPortable | cudaHostAllocMapped));
-        cell_slots().push_back(s);
-        for (size_t at = 0; at < (64 << 10); at += kCellBytes)
-            free_cells().push_back((double *)((char *)s + at));
+    Pinned &P = pinned();
+    std::lock_guard<std::mutex> lk(P.mu);
+    if (P.free_cells.empty()) {
+        void *b = P.make(kCellBlock);
+        P.blocks.push_back(b);
+        for (size_t at = 0; at < kCellBlock; at += kCellBytes)
+            P.free_cells.push_back((double *)((char *)b + at));
     }
-    p = free_cells().back();
-    free_cells().pop_back();
-    ++g_cells;
+    p = P.free_cells.back();
+    P.free_cells.pop_back();
+    ++P.cells;
     *p = 0;
 }
 
 PinnedCell::~PinnedCell()
 {
-    std::lock_guard<std::mutex> lk(slot_mu());
-    free_cells().push_back(p);
-    if (--g_cells > 0) return;
-    free_cells().clear();
-    for (void *s : cell_slots()) cudaFreeHost(s);
-    cell_slots().clear();
+    Pinned &P = pinned();
+    std::lock_guard<std::mutex> lk(P.mu);
+    P.free_cells.push_back(p);
+    --P.cells;
 }
 
 namespace {

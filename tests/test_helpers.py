@@ -35,3 +35,12 @@ def test_forked_child_ends(tmp_path):
     r = subprocess.run([stress(tmp_path, 60000), "0.2", "1", "fork"], stdout=subprocess.PIPE, text=True,
                        timeout=60)
     assert r.returncode == 0, r.stdout
+
+
+def test_given_back_once_unused(tmp_path):
+    exe = str(tmp_path / "give_back")
+    subprocess.run(["g++", "-std=c++17", "-O2", "-pthread", "-DNADIA_HELPER_LINGER_MS=200", "-I", CSRC,
+                    os.path.join(ROOT, "tests", "helpers_give_back.cpp"),
+                    os.path.join(CSRC, "helpers.cpp"), "-o", exe], check=True)
+    r = subprocess.run([exe], stdout=subprocess.PIPE, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout
