@@ -12,7 +12,6 @@
 #include <condition_variable>
 #include <deque>
 #include <mutex>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -27,6 +26,8 @@ namespace nadia {
 namespace {
 using Clock = std::chrono::steady_clock;
 constexpr std::chrono::milliseconds kHelperLinger{NADIA_HELPER_LINGER_MS};
+// as many as there are pinned slots; half the cores where those are fewer
+constexpr int kMostHelpers = 16;
 
 // one with_helpers call: helpers it still wants, and those at work in it
 struct Task {
@@ -41,6 +42,8 @@ struct Helpers {
     std::vector<std::thread> ended;   // to be joined, which does not wait
     std::deque<Task *> tasks;
     std::vector<void (*)()> give_back; // by the last helper to end
+    int asleep = 0, starting = 0; // helpers not at work
+    int wanted = 0;               // those that the tasks still want
     size_t uses = 0;
     Clock::time_point unused_since = Clock::now();
     bool closed = false; // the process (or the library) ends; never lowered
@@ -69,18 +72,23 @@ void help()
     Helpers &h = helpers();
     std::unique_lock<std::mutex> lk(h.mu);
     bool given = false;
+    --h.starting;
     for (;;) {
         if (h.closed) return;
         if (h.tasks.empty()) {
             const Clock::time_point until = h.unused_since + kHelperLinger;
             if (h.uses > 0) {
                 given = false;
+                ++h.asleep;
                 h.wake.wait(lk);
+                --h.asleep;
                 continue;
             }
             if (Clock::now() < until) {
                 given = false;
+                ++h.asleep;
                 h.wake.wait_until(lk, until);
+                --h.asleep;
                 continue;
             }
             // unused for long enough
@@ -102,6 +110,7 @@ void help()
             return;
         }
         Task *t = h.tasks.front();
+        --h.wanted;
         if (--t->want == 0) h.tasks.pop_front();
         ++t->running;
         lk.unlock();
@@ -109,6 +118,13 @@ void help()
         lk.lock();
         if (--t->running == 0) h.done.notify_all();
     }
+}
+
+// one helper more, with h.mu held
+void start(Helpers &h)
+{
+    h.threads.emplace_back(help);
+    ++h.starting;
 }
 
 // the helpers that have ended, with h.mu held (they hold it no more)
@@ -153,7 +169,7 @@ HelperUse::~HelperUse()
         h.unused_since = Clock::now();
         try {
             // there is one to give things back
-            if (!h.closed && h.threads.empty() && !h.give_back.empty()) h.threads.emplace_back(help);
+            if (!h.closed && h.threads.empty() && !h.give_back.empty()) start(h);
         } catch (...) {
             // they stay until the next time
         }
@@ -170,7 +186,7 @@ void when_unused(void (*give_back)())
 
 void with_helpers(int extra, const std::function<void()> &f)
 {
-    static const int most = (int)std::thread::hardware_concurrency() / 2;
+    static const int most = std::min((int)std::thread::hardware_concurrency() / 2, kMostHelpers);
     extra = std::min(extra, most);
     if (extra <= 0) {
         f();
@@ -180,24 +196,26 @@ void with_helpers(int extra, const std::function<void()> &f)
     Task t{&f, extra, 0};
     {
         std::lock_guard<std::mutex> lk(h.mu);
-        if (h.closed) t.want = 0;
-        try {
-            reap(h);
-            while (!h.closed && (int)h.threads.size() < most) h.threads.emplace_back(help);
-        } catch (const std::system_error &) {
-            // fewer helpers then
+        if (h.closed) {
+            t.want = 0;
+        } else {
+            h.tasks.push_back(&t);
+            h.wanted += extra;
+            try {
+                reap(h);
+                while (h.asleep + h.starting < h.wanted && (int)h.threads.size() < most) start(h);
+            } catch (...) {
+                // fewer helpers then
+            }
         }
-        if (t.want > 0) h.tasks.push_back(&t);
     }
-    if (extra == 1)
-        h.wake.notify_one();
-    else
-        h.wake.notify_all();
+    for (int k = 0; k < extra; ++k) h.wake.notify_one();
     f();
     std::unique_lock<std::mutex> lk(h.mu);
     for (auto it = h.tasks.begin(); it != h.tasks.end(); ++it)
         if (*it == &t) {
             h.tasks.erase(it);
+            h.wanted -= t.want;
             break;
         }
     h.done.wait(lk, [&] { return t.running == 0; });

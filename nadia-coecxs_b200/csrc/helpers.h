@@ -17,9 +17,9 @@ public:
 
 // Runs f on the calling thread and on up to `extra` helper threads at once;
 // returns when all have returned.  f divides its work among its callers itself
-// and does not throw.  The helpers are the process's (half its cores at most,
-// shared by all concurrent calls; starting threads for each call instead cost
-// about 0.1 ms).
+// and does not throw.  The helpers are the process's, shared by all concurrent
+// calls and started as calls want them, up to sixteen or half the cores; starting
+// threads for each call instead cost about 0.1 ms.
 void with_helpers(int extra, const std::function<void()> &f);
 
 // give_back() is called on a helper thread when there has been no reconstruction

@@ -44,3 +44,15 @@ def test_given_back_once_unused(tmp_path):
                     os.path.join(CSRC, "helpers.cpp"), "-o", exe], check=True)
     r = subprocess.run([exe], stdout=subprocess.PIPE, text=True, timeout=60)
     assert r.returncode == 0, r.stdout
+
+
+# helpers wanted by a call, calls at once, and the most helpers that may run
+@pytest.mark.parametrize("extra,calls,most", [(1, 1, 1), (2, 1, 2), (7, 1, 7), (7, 4, 16)])
+def test_started_as_wanted(tmp_path, extra, calls, most):
+    exe = str(tmp_path / "count")
+    subprocess.run(["g++", "-std=c++17", "-O2", "-pthread", "-I", CSRC,
+                    os.path.join(ROOT, "tests", "helpers_count.cpp"),
+                    os.path.join(CSRC, "helpers.cpp"), "-o", exe], check=True)
+    r = subprocess.run([exe, str(extra), str(calls)], stdout=subprocess.PIPE, text=True, timeout=60)
+    assert r.returncode == 0
+    assert min(1, os.cpu_count() // 2) <= int(r.stdout) <= min(most, max(1, os.cpu_count() // 2)), r.stdout
