@@ -209,7 +209,10 @@ void with_helpers(int extra, const std::function<void()> &f)
             }
         }
     }
-    for (int k = 0; k < extra; ++k) h.wake.notify_one();
+    if (extra == 1)
+        h.wake.notify_one();
+    else
+        h.wake.notify_all(); // one call of the kernel; there are sixteen at most
     f();
     std::unique_lock<std::mutex> lk(h.mu);
     for (auto it = h.tasks.begin(); it != h.tasks.end(); ++it)
