@@ -935,7 +935,7 @@ void put_rows(const T *h, void *dst, bool fold, int nx, int ny, int device,
     constexpr int q = kPanel * stride; // values of a panel row
     const int np = ny / kPanel;
     const size_t run = (size_t)q * sizeof(float);
-    in_pieces(device, st, nx, w * sizeof(float), [&](CopySlot &slot, size_t r0, size_t rows) {
+    in_pieces(device, st, nullptr, 0, nx, w * sizeof(float), [&](CopySlot &slot, size_t r0, size_t rows) {
         float *p = static_cast<float *>(slot.p);
         for (size_t x = 0; x < rows; ++x) {
             // row x of the piece is row r0 + x of the device array
@@ -962,7 +962,8 @@ void get_rows(const void *src, T *h, int nx, int ny, int device, cudaStream_t st
     constexpr int q = kPanel * stride;
     const int np = ny / kPanel;
     const size_t run = (size_t)q * sizeof(float);
-    in_pieces(device, st, nx, w * sizeof(float), [&](CopySlot &slot, size_t r0, size_t rows) {
+    in_pieces(device, st, h, nx * w * sizeof(T), nx, w * sizeof(float), [&](CopySlot &slot, size_t r0,
+                                                                            size_t rows) {
         const float *p = static_cast<const float *>(slot.p);
         NADIA_CUDA(cudaMemcpy2DAsync(slot.p, rows * run, (const char *)src + r0 * run,
                                      (size_t)nx * run, rows * run, np, cudaMemcpyDeviceToHost, st));

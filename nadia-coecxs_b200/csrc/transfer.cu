@@ -140,6 +140,39 @@ constexpr size_t kRow = 64 << 10;      // plain copies are cut in "rows" of this
 constexpr size_t kSmallCopy = 2 << 20; // below: the driver's own staging (about 16 GB/s)
 } // namespace
 
+void await(cudaStream_t st, void *fill, size_t bytes)
+{
+    {
+        NoCapture guard;
+        const cudaError_t ready = cudaStreamQuery(st);
+        if (ready == cudaSuccess) return; // no wait to hide anything behind
+        if (ready == cudaErrorNotReady) (void)cudaGetLastError();
+        else NADIA_CUDA(ready);
+    }
+    if (!fill) {
+        NADIA_CUDA(cudaStreamSynchronize(st));
+        return;
+    }
+    constexpr size_t kTouch = 64 << 10, kPage = 4096;
+    std::atomic<size_t> next{0};
+    std::atomic<bool> over{false};
+    cudaError_t e = cudaSuccess;
+    const std::thread::id caller = std::this_thread::get_id();
+    with_helpers((int)std::min<size_t>(7, bytes / (4 * kTouch)), [&] {
+        if (std::this_thread::get_id() == caller) {
+            e = cudaStreamSynchronize(st);
+            over = true;
+            return;
+        }
+        for (size_t at; !over && (at = next.fetch_add(kTouch)) < bytes;)
+            for (size_t k = at; k < std::min(bytes, at + kTouch); k += kPage) {
+                volatile char *p = (char *)fill + k;
+                *p = *p; // a write, so that the page becomes the array's own
+            }
+    });
+    NADIA_CUDA(e);
+}
+
 void to_device(void *d, const void *h, size_t bytes, int device, cudaStream_t st)
 {
     if (bytes < kSmallCopy) {
@@ -147,7 +180,8 @@ void to_device(void *d, const void *h, size_t bytes, int device, cudaStream_t st
         NADIA_CUDA(cudaStreamSynchronize(st));
         return;
     }
-    in_pieces(device, st, (bytes + kRow - 1) / kRow, kRow, [&](CopySlot &slot, size_t r, size_t rows) {
+    in_pieces(device, st, nullptr, 0, (bytes + kRow - 1) / kRow, kRow, [&](CopySlot &slot, size_t r,
+                                                                   size_t rows) {
         const size_t at = r * kRow, len = std::min(rows * kRow, bytes - at);
         std::memcpy(slot.p, (const char *)h + at, len);
         NADIA_CUDA(cudaMemcpyAsync((char *)d + at, slot.p, len, cudaMemcpyHostToDevice, st));
@@ -162,7 +196,8 @@ void to_host(void *h, const void *d, size_t bytes, int device, cudaStream_t st)
         NADIA_CUDA(cudaStreamSynchronize(st));
         return;
     }
-    in_pieces(device, st, (bytes + kRow - 1) / kRow, kRow, [&](CopySlot &slot, size_t r, size_t rows) {
+    in_pieces(device, st, h, bytes, (bytes + kRow - 1) / kRow, kRow, [&](CopySlot &slot, size_t r,
+                                                                 size_t rows) {
         const size_t at = r * kRow, len = std::min(rows * kRow, bytes - at);
         NADIA_CUDA(cudaMemcpyAsync(slot.p, (const char *)d + at, len, cudaMemcpyDeviceToHost, st));
         slot.wait(st);

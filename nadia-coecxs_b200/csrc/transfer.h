@@ -82,21 +82,31 @@ struct CopySlot {
     }
 };
 
+// Waits for the work queued on st.  Meanwhile helpers bring in the pages of the
+// array that a read is about to fill (null: none), which leaves its contents as
+// they are; they stop when the wait ends and never wait for it.
+void await(cudaStream_t st, void *fill, size_t bytes);
+
 // Calls body(slot, first row, rows) for pieces of `rows` rows of `row_bytes`
 // (as they pass through a slot); each piece is done when its call returns.
-// The first error of any thread is thrown once all have stopped.
+// The first error of any thread is thrown once all have stopped.  fill: the
+// array of `bytes` that a read fills, or null.
 //
-// The calling thread waits for the work queued on st before any slot or helper
-// is taken, so that those are held for copies only: a read behind long
+// The calling thread waits for the work queued on st before any slot is taken,
+// so that slots and helpers are held for copies only: a read behind long
 // iterations otherwise held eight of the sixteen slots until they ended, and a
 // few such reads kept every other reconstruction's transfers waiting (and each
-// of their threads polling) although its own stream was idle.
+// of their threads polling) although its own stream was idle.  While
+// it waits, helpers bring in the pages of a fresh array: B200, reads right behind
+// iterations, 2048^2: FP64 3.5 -> 2.1 ms, FP32 2.1 -> 1.8 ms, 512^2 FP32 0.20 ms
+// either way.
 template <class Body>
-void in_pieces(int device, cudaStream_t st, size_t rows, size_t row_bytes, Body body)
+void in_pieces(int device, cudaStream_t st, void *fill, size_t bytes, size_t rows, size_t row_bytes,
+               Body body)
 {
     NADIA_REQUIRE(row_bytes <= kSlotBytes, NADIA_ERR_INVALID, "row too long to transfer");
     if (rows == 0) return;
-    NADIA_CUDA(cudaStreamSynchronize(st));
+    await(st, fill, bytes);
     const size_t fit = kSlotBytes / row_bytes;
     // two pieces a thread at least, and pieces worth a thread's start
     const size_t worth = std::max<size_t>(1, (1u << 20) / row_bytes);
