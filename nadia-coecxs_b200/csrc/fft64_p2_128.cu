@@ -16,7 +16,6 @@ bool cols_p2_128(int L, ColMode mode, bool fwd, const Fft64Args &A, cudaStream_t
 {
     switch (L) {
     case 4: return cols_modes<128, 4>(mode, fwd, A, st);
-    case 8: return cols_modes<128, 8>(mode, fwd, A, st);
     default: return false;
     }
 }

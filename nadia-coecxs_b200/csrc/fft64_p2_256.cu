@@ -19,7 +19,6 @@ bool cols_p2_256(int L, ColMode mode, bool fwd, const Fft64Args &A, cudaStream_t
     switch (L) {
     case 2: return cols_modes<256, 2>(mode, fwd, A, st);
     case 4: return cols_modes<256, 4>(mode, fwd, A, st);
-    case 8: return cols_modes<256, 8>(mode, fwd, A, st);
     default: return false;
     }
 }

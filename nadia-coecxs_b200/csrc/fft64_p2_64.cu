@@ -8,7 +8,6 @@ bool rows_p2_64(int L, RowMode mode, bool fwd, const Fft64Args &A, cudaStream_t 
 {
     switch (L) {
     case 4: return rows_modes<64, 4>(mode, fwd, A, st);
-    case 8: return rows_modes<64, 8>(mode, fwd, A, st);
     default: return false;
     }
 }
@@ -17,7 +16,6 @@ bool cols_p2_64(int L, ColMode mode, bool fwd, const Fft64Args &A, cudaStream_t 
 {
     switch (L) {
     case 4: return cols_modes<64, 4>(mode, fwd, A, st);
-    case 8: return cols_modes<64, 8>(mode, fwd, A, st);
     default: return false;
     }
 }

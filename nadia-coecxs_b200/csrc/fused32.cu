@@ -1015,7 +1015,7 @@ void Fused32::Impl::flush_intensity()
 {
     if (!mI_dirty) return;
     mI_dirty = false;
-    std::vector<float> &m = mstage; // kept between calls, like the staging array
+    std::vector<float> &m = mstage; // kept between calls
     m.resize(n);
     // the sum by fixed parts, added in order (the same on every machine)
     std::vector<double> sums((n + kPart - 1) / kPart, 0.0);

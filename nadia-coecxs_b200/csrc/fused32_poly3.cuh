@@ -225,18 +225,17 @@ __global__ void __launch_bounds__(T::NT, T::MINB) k_poly3_row(const Slot *const 
     if (MODE == kRowFull) {
         float2 *xs = sm + T::N * T::L;
         float *ss = reinterpret_cast<float *>(xs + T::N * T::L);
-        const bool staged = (ny & 3) == 0, er = S.er;
-        if (staged) {
-            // the tile's rows of a panel are one run of 16 elements
-            const int nseg = ny / kPanel;
-            const float2 *__restrict__ xg = x + (size_t)i0 * kPanel;
-            const float *__restrict__ sg = S.sup + (size_t)i0 * kPanel;
-            if (!er)
-                for (int c = threadIdx.x; c < nseg * 8; c += T::NT)
-                    cp_async16(xs + c * 2, xg + (size_t)(c / 8) * nx * kPanel + 2 * (c % 8));
-            for (int c = threadIdx.x; c < nseg * 4; c += T::NT)
-                cp_async16(ss + c * 4, sg + (size_t)(c / 4) * nx * kPanel + 4 * (c % 4));
-        }
+        const bool er = S.er;
+        // the tile's rows of a panel are one run of 16 elements (ny is a multiple
+        // of four in this form)
+        const int nseg = ny / kPanel;
+        const float2 *__restrict__ xg = x + (size_t)i0 * kPanel;
+        const float *__restrict__ sg = S.sup + (size_t)i0 * kPanel;
+        if (!er)
+            for (int c = threadIdx.x; c < nseg * 8; c += T::NT)
+                cp_async16(xs + c * 2, xg + (size_t)(c / 8) * nx * kPanel + 2 * (c % 8));
+        for (int c = threadIdx.x; c < nseg * 4; c += T::NT)
+            cp_async16(ss + c * 4, sg + (size_t)(c / 4) * nx * kPanel + 4 * (c % 4));
         if (blockIdx.x == 0 && S.project) {
             double t = 0.0;
             for (int b = threadIdx.x; b < S.ncol; b += T::NT) t += S.partials[b];
@@ -257,11 +256,8 @@ __global__ void __launch_bounds__(T::NT, T::MINB) k_poly3_row(const Slot *const 
             v[e] = P[paddr(px + i0 + s, pos, mx)];
         });
         transform3<T, kRowMap, false>(v, sm, tw);
-        if (staged) {
-            cp_async_wait_all();
-            __syncthreads();
-        }
-        const float *__restrict__ sup = S.sup;
+        cp_async_wait_all();
+        __syncthreads();
         const float wid = S.w_id, wpf = S.w_pf, wps = S.w_ps, wpsf = S.w_psf;
         each3<T, kRowMap, T::RC>([&](int e, int s, int pos) {
             const int j = pos - py;
@@ -269,11 +265,11 @@ __global__ void __launch_bounds__(T::NT, T::MINB) k_poly3_row(const Slot *const 
             if (j >= 0 && j < ny) {
                 const size_t a = paddr(i0 + s, j, nx);
                 const int b = (j / kPanel * T::L + s) * kPanel + j % kPanel; // staged index
-                const float f = support_factor(staged ? ss[b] : __ldg(&sup[a]));
+                const float f = support_factor(ss[b]);
                 if (er)
                     xn = cscale(v[e], f);
                 else
-                    xn = combine2(staged ? xs[b] : x[a], v[e], f, wid, wpf, wps, wpsf);
+                    xn = combine2(xs[b], v[e], f, wid, wpf, wps, wpsf);
                 x[a] = xn;
             }
             v[e] = xn;

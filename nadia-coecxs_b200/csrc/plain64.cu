@@ -146,34 +146,20 @@ __device__ __forceinline__ double2 supported(double2 v, double sv)
     return v;
 }
 
-// The combine loop with the support projections formed on the fly (no
-// transmission constraint, no PfPs term): Ps x = support(x), PsPf x =
-// support(Pf x); the same sums in the same order as copying, projecting and
-// combining separately.
-__global__ void k_combine_support(double2 *x, const double2 *__restrict__ pf,
-                                  const double *__restrict__ sup, int use_ps, int use_psf,
-                                  Weights W, size_t n)
+// The combine loop with Ps x = support(x) formed on the fly (no transmission
+// constraint, no other projection); the same sums in the same order as copying,
+// projecting and combining separately.
+__global__ void k_combine_support(double2 *x, const double *__restrict__ sup, int use_ps, Weights W,
+                                  size_t n)
 {
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n;
          k += (size_t)gridDim.x * blockDim.x) {
         const double2 v = x[k];
-        const double sv = sup[k];
         double vr = W.id * v.x, vi = W.id * v.y;
-        double2 f = make_double2(0.0, 0.0);
-        if (pf) {
-            f = pf[k];
-            vr += W.w[3] * f.x;
-            vi += W.w[3] * f.y;
-        }
         if (use_ps) {
-            const double2 t = supported(v, sv);
+            const double2 t = supported(v, sup[k]);
             vr += W.w[2] * t.x;
             vi += W.w[2] * t.y;
-        }
-        if (use_psf) {
-            const double2 t = supported(f, sv);
-            vr += W.w[0] * t.x;
-            vi += W.w[0] * t.y;
         }
         x[k] = make_double2(vr, vi);
     }
@@ -633,14 +619,13 @@ void combine(double2 *x, const double2 *pfs, const double2 *pf, const double2 *p
     k_combine<<<grid_of(n), kThreads, 0, s>>>(x, pfs, pf, ps, psf, W, n);
 }
 
-void combine_support(double2 *x, const double2 *pf, const double *support, bool use_ps,
-                     bool use_psf, const double w[5], size_t n, cudaStream_t s)
+void combine_support(double2 *x, const double *support, bool use_ps, const double w[5], size_t n,
+                     cudaStream_t s)
 {
     Weights W;
     for (int i = 0; i < 5; ++i) W.w[i] = w[i];
     W.id = 1 + w[4];
-    k_combine_support<<<grid_of(n), kThreads, 0, s>>>(x, pf, support, use_ps ? 1 : 0,
-                                                     use_psf ? 1 : 0, W, n);
+    k_combine_support<<<grid_of(n), kThreads, 0, s>>>(x, support, use_ps ? 1 : 0, W, n);
 }
 
 void multiply_factors(double2 *c, const double2 *coef, int nx, int ny, int direction,

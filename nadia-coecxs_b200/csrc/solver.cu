@@ -309,7 +309,7 @@ void Solver::set_spectrum(const double *wl_weight, int nl)
 
 // The sample row and column of each line for every measured pixel, in the
 // operation order of expand_wl (PolyCDI.c++:312-318); -1 outside the padded
-// grid.  Rows are kept as offsets into the padded array.
+// grid.
 void Solver::poly_tables()
 {
     const int mx = nx + 2 * px, my = ny + 2 * py;
@@ -1198,8 +1198,8 @@ void Solver::fused64_iterate()
 }
 
 // BaseCDI::iterate, BaseCDI.c++:297-387; PolyCDI::iterate, PolyCDI.c++:130-250
-// -- the forms fused64_iterate leaves: transmission constraints and algorithms
-// with the PfPs term
+// -- the forms fused64_iterate leaves: transmission constraints, algorithms with
+// the PfPs term and algorithms without the Pf term
 void Solver::plain_iterate_once()
 {
     AllocScope scope(st);
@@ -1217,16 +1217,9 @@ void Solver::plain_iterate_once()
         plain_apply_support(x.p);
         return;
     }
-    if (!tc.active && w[PFS] == 0 && (w[PSF] == 0 || w[PF] != 0)) {
-        // the support projections formed inside the combine (same arithmetic)
-        const bool pf = w[PF] != 0;
-        if (pf) {
-            if (!tPF) tPF.alloc(n);
-            NADIA_CUDA(cudaMemcpyAsync(tPF.p, x.p, nb, cudaMemcpyDeviceToDevice, st));
-            plain_project(tPF.p);
-        }
-        plain::combine_support(x.p, pf ? tPF.p : nullptr, support.p, w[PS] != 0, w[PSF] != 0,
-                               w, n, st);
+    if (!tc.active && w[PFS] == 0 && w[PSF] == 0) {
+        // no projection onto the intensity (fused64_iterate has those with Pf)
+        plain::combine_support(x.p, support.p, w[PS] != 0, w, n, st);
         return;
     }
     ensure_temps();

@@ -82,7 +82,7 @@ struct Solver {
     DevBuf<double> d_spec, isc;
     DevBuf<double2> padded;
     DevBuf<double> d_q;           // |Psi|^2 of the centred padded field
-    DevBuf<int> d_rows, d_cols;   // sample rows (as offsets) and columns of each line
+    DevBuf<int> d_rows, d_cols;   // sample rows and columns of each line (-1: outside)
     plain::Fft2d fft_pad;
 
     // TransmissionConstraint set by BaseCDI::set_complex_constraint (FP64 form)
