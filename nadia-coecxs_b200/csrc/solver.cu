@@ -875,6 +875,7 @@ void Solver::convert_to_fp64()
         h2d(illum.p, h_illum.data(), illum.bytes(), st);
         fresnel_set_experimental_parameters(wavelength, zfd, zfs, pixel);
     }
+    if (kind == NADIA_FRESNEL_WF) fresnel_wf_init(wavelength, z12, z23, pixel);
     if (kind == NADIA_POLY && has_spectrum) {
         d_spec.alloc(2 * (size_t)nlambda);
         h2d(d_spec.p, spectrum.data(), d_spec.bytes(), st);
