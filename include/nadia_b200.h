@@ -140,10 +140,10 @@ int nadia_read_spec(const char *path, double *rows, int capacity, int *nrows);
 
 /* Moves an FP32 reconstruction to the FP64 form in place (no-op on FP64):
  * estimate, support, intensity, beam stop, Fresnel illumination and geometry,
- * spectrum, algorithm, error history and n-best results carry over, FP32
- * values widened.  Needed before complex-constraint regions or a custom
- * constraint function (FP64 only), or any constraint or phase-diverse
- * position on an FP32 PolyCDI. */
+ * spectrum, algorithm, transmission constraint with its regions, error history
+ * and n-best results carry over, FP32 values widened.  Needed before a custom
+ * constraint function (FP64 only), or any constraint or phase-diverse position
+ * on an FP32 PolyCDI. */
 int nadia_convert_to_fp64(nadia_solver *s);
 
 /* NADIA_FP32 or NADIA_FP64. */
@@ -164,10 +164,10 @@ int nadia_poly_get_padding(const nadia_solver *s, int *px, int *py);
  * most 16) ComplexConstraint regions, given as nregions masks of nx*ny
  * (a pixel belongs to the first region whose mask is > 0 there), alpha as
  * nregions pairs (alpha1, alpha2), fixed_c as nregions values (NaN = c_mean
- * measured each time; NULL = all measured).  The FP32 form runs the
- * per-pixel part (unit magnitude, charge flipping) inside its fused row pass
- * and returns NADIA_ERR_UNSUPPORTED for regions and for PolyCDI: convert the
- * handle first (nadia_convert_to_fp64). */
+ * measured each time; NULL = all measured).  The FP32 form runs it inside its
+ * fused row pass (split around the regions' sums) and returns
+ * NADIA_ERR_UNSUPPORTED for PolyCDI: convert the handle first
+ * (nadia_convert_to_fp64). */
 int nadia_set_transmission_constraint(nadia_solver *s, int enforce_unity, int charge_flip,
                                       int flip_sign, int nregions, const double *regions,
                                       const double *alpha, const double *fixed_c);

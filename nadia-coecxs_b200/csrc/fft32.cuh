@@ -43,11 +43,11 @@ __device__ __forceinline__ void let_next_start()
 // with separate products Dft<3> was 17% and Dft<8> 3.5% further from 64 bits
 // (root mean square, 4.09e-8 -> 4.79e-8 and 8.83e-8 -> 9.14e-8).  The passes
 // are bound by instruction issue, and sums and differences of complex values
-// are half of a transform's arithmetic: FresnelCDI 2048^2 86.5 -> 80.9 us an
-// iteration, five sizes batched 248 -> 230, 16 PlanarCDI 2048^2 884 -> 861,
-// PolyCDI 1024^2 x 4 197.5 -> 189 (B200).  FresnelCDI_WF's passes keep the
-// scalar form (2048^2 122.6 us against 131 packed: four transforms in a kernel,
-// out of registers for the pairs).
+// are half of a transform's arithmetic (B200, scalar, packed, and packed with
+// those multiply-adds): FresnelCDI 2048^2 86.5, 80.9 and 80.6 us an iteration,
+// five sizes batched 248, 239 and 235, 16 PlanarCDI 2048^2 884, 874 and 862.
+// FresnelCDI_WF's passes keep the scalar form (2048^2 120 us against 131 packed:
+// four transforms in a kernel, out of registers for the pairs).
 template <bool PK = true>
 __device__ __forceinline__ float2 cadd(float2 a, float2 b)
 {

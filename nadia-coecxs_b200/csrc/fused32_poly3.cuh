@@ -9,9 +9,9 @@
 // value of a thread through all passes need 6*6*6*5 with 30 values, 168
 // registers and ten warps, too few to hide the loads and the exchanges.
 // B200, PolyCDI 1024^2 padded to 1080^2, an iteration: one reconstruction 49.9 us
-// with those tiles and 40.1 with these, four 189 and 138, eight 359 and 275.
-// Forming two thirds of the twiddles as products, as the other tiles do, takes
-// four to 134 us but leaves the estimate 1.9e-6 from 64 bits after 32 HIO
+// with those tiles and 39.1 with these, four 189 and 135, eight 359 and 271.
+// Forming two thirds of the twiddles as products, as the other tiles do, took
+// four from 138 to 134 us but leaves the estimate 1.9e-6 from 64 bits after 32 HIO
 // iterations, against 1.7e-6 for those tiles and 1.0e-6 with every twiddle from
 // the table.
 //

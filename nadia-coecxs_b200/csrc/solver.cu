@@ -440,46 +440,13 @@ void Solver::set_transmission_constraint(int unity, int flip, int flip_sign, int
                   "between 0 and 16 complex-constraint regions");
     NADIA_REQUIRE(nregions == 0 || n % 4 == 0, NADIA_ERR_UNSUPPORTED,
                   "complex-constraint regions need a pixel count divisible by 4");
-    if (prec == NADIA_FP32) {
-        // the per-pixel part runs inside the fused row pass; regions split
-        // the row pass around their sums (fused32_tc.cuh)
-        NADIA_REQUIRE(kind != NADIA_POLY, NADIA_ERR_UNSUPPORTED,
-                      "PolyCDI constraints run in the FP64 form: convert the reconstruction "
-                      "first");
-        NADIA_REQUIRE(nregions == 0 || (regions && alpha), NADIA_ERR_INVALID,
-                      "complex-constraint regions need their masks and alphas");
-        std::vector<int> map(nregions > 0 ? n : 0, 0);
-        std::vector<double> prm(4 * (size_t)nregions, 0.0);
-        for (int r = 0; r < nregions; ++r) {
-            for (size_t k = 0; k < n; ++k)
-                if (regions[(size_t)r * n + k] > 0 && map[k] == 0) map[k] = r + 1;
-            prm[4 * r] = alpha[2 * r];
-            prm[4 * r + 1] = alpha[2 * r + 1];
-            const bool fixed = fixed_c && fixed_c[r] == fixed_c[r];
-            prm[4 * r + 2] = fixed ? 1.0 : 0.0;
-            prm[4 * r + 3] = fixed ? fixed_c[r] : 0.0;
-        }
-        f32->set_constraint(true, unity != 0, flip != 0, flip_sign, nregions, map.data(),
-                            prm.data());
-        tc.active = true;
-        tc.unity = unity ? 1 : 0;
-        tc.flip = flip ? 1 : 0;
-        tc.flip_sign = flip_sign > 0 ? 1 : -1;
-        tc.nregions = nregions;
-        tc.custom = nullptr;
-        tc.user = nullptr;
-        return;
-    }
+    // PolyCDI's rows are transformed on the padded grid, without a place for it
+    NADIA_REQUIRE(prec == NADIA_FP64 || kind != NADIA_POLY, NADIA_ERR_UNSUPPORTED,
+                  "PolyCDI constraints run in the FP64 form: convert the reconstruction first");
     NADIA_REQUIRE(nregions == 0 || (regions && alpha), NADIA_ERR_INVALID,
                   "complex-constraint regions need their masks and alphas");
-    NADIA_CUDA(cudaStreamSynchronize(st)); // buffers of an earlier constraint may be replaced
-    tc.active = true;
-    tc.unity = unity ? 1 : 0;
-    tc.flip = flip ? 1 : 0;
-    tc.flip_sign = flip_sign > 0 ? 1 : -1;
-    tc.nregions = nregions;
-    std::vector<int> map(n, 0);
-    std::vector<double> prm(4 * (size_t)std::max(nregions, 1), 0.0);
+    std::vector<int> map(nregions > 0 ? n : 0, 0);
+    std::vector<double> prm(4 * (size_t)nregions, 0.0);
     for (int r = 0; r < nregions; ++r) {
         for (size_t k = 0; k < n; ++k)
             if (regions[(size_t)r * n + k] > 0 && map[k] == 0) map[k] = r + 1;
@@ -489,10 +456,39 @@ void Solver::set_transmission_constraint(int unity, int flip, int flip_sign, int
         prm[4 * r + 2] = fixed ? 1.0 : 0.0;
         prm[4 * r + 3] = fixed ? fixed_c[r] : 0.0;
     }
+    // the per-pixel part runs inside the fused row pass; regions split the row
+    // pass around their sums (fused32_tc.cuh)
+    if (prec == NADIA_FP32)
+        f32->set_constraint(true, unity != 0, flip != 0, flip_sign, nregions, map.data(),
+                            prm.data());
+    else
+        NADIA_CUDA(cudaStreamSynchronize(st)); // buffers of an earlier constraint may be replaced
+    tc.active = true;
+    tc.unity = unity ? 1 : 0;
+    tc.flip = flip ? 1 : 0;
+    tc.flip_sign = flip_sign > 0 ? 1 : -1;
+    tc.nregions = nregions;
+    if (prec == NADIA_FP32) {
+        // kept for convert_to_fp64
+        tc.map = std::move(map);
+        tc.prm = std::move(prm);
+        tc.custom = nullptr;
+        tc.user = nullptr;
+        return;
+    }
+    upload_constraint(map, prm);
+}
+
+// FP64: the constraint's buffers (map: each pixel's region, empty without any)
+void Solver::upload_constraint(std::vector<int> map, std::vector<double> prm)
+{
+    const size_t R = (size_t)std::max(tc.nregions, 1);
+    map.resize(n, 0);
+    prm.resize(4 * R, 0.0);
     tc.region.alloc(n);
     tc.params.alloc(prm.size());
-    tc.partials.alloc(2 * (size_t)plain::kRedBlocks * std::max(nregions, 1));
-    tc.cmean.alloc(std::max(nregions, 1));
+    tc.partials.alloc(2 * (size_t)plain::kRedBlocks * R);
+    tc.cmean.alloc(R);
     if (kind == NADIA_FRESNEL && !tc.tbuf) tc.tbuf.alloc(n);
     h2d(tc.region.p, map.data(), n * sizeof(int), st);
     h2d(tc.params.p, prm.data(), prm.size() * sizeof(double), st);
@@ -842,8 +838,7 @@ void Solver::convert_to_fp64()
     forget_batches_with(uid); // batch plans hold FP32 handles only
     NADIA_CUDA(cudaStreamSynchronize(st));
     const bool had_tc = tc.active;
-    const int tcu = tc.unity, tcf = tc.flip, tcs = tc.flip_sign;
-    tc.active = false;
+    tc.active = false; // until its FP64 buffers are made
     f32.reset();
     best32.clear();
     prec = NADIA_FP64;
@@ -884,7 +879,8 @@ void Solver::convert_to_fp64()
         fft_pad.init(nx + 2 * px, ny + 2 * py);
         poly_tables();
     }
-    if (had_tc) set_transmission_constraint(tcu, tcf, tcs, 0, nullptr, nullptr, nullptr);
+    if (had_tc) upload_constraint(std::move(tc.map), std::move(tc.prm));
+    tc.active = had_tc;
     NADIA_CUDA(cudaStreamSynchronize(st));
 }
 

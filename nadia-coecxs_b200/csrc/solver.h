@@ -94,6 +94,8 @@ struct Solver {
         DevBuf<double> partials;  // region sums per reduction block
         DevBuf<double> cmean;     // per region
         DevBuf<double2> tbuf;     // FresnelCDI: the transmission function being constrained
+        std::vector<int> map;     // FP32: the regions as set, kept for convert_to_fp64
+        std::vector<double> prm;
         void (*custom)(double *, int, int, void *) = nullptr;
         void *user = nullptr;
     } tc;
@@ -162,6 +164,7 @@ struct Solver {
     void plain_propagate_from(double2 *c, bool padded_grid);
     void plain_scale(double2 *c);
     void plain_apply_support(double2 *c);
+    void upload_constraint(std::vector<int> map, std::vector<double> prm);
     void apply_transmission_constraint(double2 *t);
 
     // The result a PhaseDiverseCDI exchanges with this reconstruction
