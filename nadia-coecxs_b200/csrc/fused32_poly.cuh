@@ -212,9 +212,10 @@ __global__ void __launch_bounds__(C::NT, C::MINB) k_poly_col_inv(const Slot *con
         const int i = centred(kx, mx) - px, j = centred(ky, my) - py;
         float r = 1.f;
         if (i >= 0 && i < nx && j >= 0 && j < ny) r = __ldg(&ratio[paddr(i, j, nx)]);
-        v[e] = cscale(P[paddr(kx, ky, mx)], s02 * r);
+        v[e] = cscale<false>(P[paddr(kx, ky, mx)], s02 * r);
     });
-    transform<C, false>(v, sm, tw);
+    // scalar sums: the compiler contracts these products into the first ones
+    transform<Scalar<C>, false>(v, sm, tw);
     let_next_start();
     for_each_slot<C, false, false>([&](int e, int s, int pos) {
         if (pos >= px && pos < px + nx) P[paddr(pos, c0 * kPanel + s, mx)] = v[e];
